@@ -591,8 +591,11 @@ int shainet_attn_ctx_destroy(shainet_attn_ctx* c) {
     if (c->live_caches != 0) return fail(SHAINET_ATTN_E_STATE, "%d caches still alive", c->live_caches);
     DeviceGuard g(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (DevBuf* b : {&c->q_rot, &c->part, &c->part_words, &c->dev_in, &c->dev_out, &c->kv_f32})
+    for (DevBuf* b : {&c->q_rot, &c->part, &c->part_words, &c->dev_in, &c->dev_out, &c->kv_f32, &c->planes, &c->gemm_part, &c->gate_up})
         if (b->p) cudaFree(b->p);
+    for (DevBuf& b : c->act)
+        if (b.p) cudaFree(b.p);
+    if (c->planes_ev) cudaEventDestroy(c->planes_ev);
     if (c->pin_in) cudaFreeHost(c->pin_in);
     if (c->pin_out) cudaFreeHost(c->pin_out);
     if (c->status_host) cudaFreeHost(c->status_host);
@@ -647,7 +650,8 @@ int shainet_attn_ctx_timing_read(shainet_attn_ctx* c, double* total_ms, int* lau
 
 size_t shainet_attn_ctx_scratch_bytes(shainet_attn_ctx* c) {
     if (!c) return 0;
-    return (c->q_rot.cap + c->part.cap + c->part_words.cap + c->dev_in.cap + c->dev_out.cap + c->kv_f32.cap) * sizeof(float);
+    return (c->q_rot.cap + c->part.cap + c->part_words.cap + c->dev_in.cap + c->dev_out.cap + c->kv_f32.cap + c->planes.cap +
+            c->gemm_part.cap + c->gate_up.cap) * sizeof(float);
 }
 
 int shainet_attn_kv_create(shainet_attn_ctx* ctx, shainet_attn_kv** out, int num_heads, int num_kv_heads,

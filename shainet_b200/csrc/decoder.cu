@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "host_state.h"
+#include "q8_gemm_tc.h"
 
 using namespace shainet;
 
@@ -36,6 +37,7 @@ struct shainet_attn_q8 {
     float* scales = nullptr;    // [N, ceil(K/32)]
     int K = 0, N = 0;
     bool owns = false;
+    Q8Maps maps;                // for the tensor-core path (maps.ok: the weight can take it)
 };
 
 struct shainet_attn_block {
@@ -46,6 +48,7 @@ struct shainet_attn_block {
     float* norm2 = nullptr;
     signed char* qkv_q = nullptr;   // the three projections stacked: [q_dim + 2 kv_dim, d_model]
     float* qkv_s = nullptr;
+    Q8Maps qkv_maps;
     const shainet_attn_q8* wo = nullptr;
     const shainet_attn_q8* gate = nullptr;
     const shainet_attn_q8* up = nullptr;
@@ -138,10 +141,113 @@ int gemv(shainet_attn_ctx* ctx, const float* x, const signed char* q, const floa
     return SHAINET_ATTN_OK;
 }
 
+// Tensor-core product of planes [3][M][K] with one or two weights (their columns beside each other) into `out`.  Where
+// the plan splits the contraction: the splits are added into `out` (defer == null), or left in ctx->gemm_part
+// [splits][M][N] for the caller, who finds their number in *defer (1: `out` is complete).
+int gemm_tc(shainet_attn_ctx* ctx, const Q8Maps* w0, const Q8Maps* w1, int M, int K, const Q8GemmOut& out, int* defer, cudaStream_t s) {
+    const int N = w0->N + (w1 ? w1->N : 0);
+    const Q8GemmPlan plan = q8_gemm_plan(M, K, w0->N, w1 ? w1->N : 0, ctx->sm_count);
+    Q8GemmArgs g{};
+    g.planes = reinterpret_cast<const __nv_bfloat16*>(ctx->planes.p);
+    g.w[0] = w0;
+    g.w[1] = w1;
+    g.M = M;
+    g.K = K;
+    g.out = out;
+    g.status = ctx->status_dev;
+    const size_t stride = (size_t)M * N;
+    if (plan.splits > 1) {
+        int rc = grow(ctx->gemm_part, stride * plan.splits, s);
+        if (rc) return rc;
+        g.out = Q8GemmOut{{ctx->gemm_part.p}, {0}, {N}, 1, stride, nullptr};
+    }
+    CU(launch_q8_gemm_tc(g, plan, ctx->sm_count, s));
+    if (defer) *defer = plan.splits;
+    else if (plan.splits > 1) CU(launch_q8_reduce(ctx->gemm_part.p, plan.splits, stride, M, N, out, s));
+    ctx->last_fused = false;
+    ctx->after_chain_kernel = true;
+    return SHAINET_ATTN_OK;
+}
+
+// Before the planes and the partials are written on stream s: the newest q8_gemv_dev call on another stream has used them.
+int planes_acquire(shainet_attn_ctx* ctx, cudaStream_t s) {
+    if (ctx->planes_pending && ctx->planes_stream != s) CU(cudaStreamWaitEvent(s, ctx->planes_ev, 0));
+    return SHAINET_ATTN_OK;
+}
+
+// Rows x [M, K] (RMS-normalised with gamma unless it is null) as the bfloat16 planes gemm_tc reads.
+int make_planes(shainet_attn_ctx* ctx, const float* x, int M, int K, const float* gamma, double eps, cudaStream_t s) {
+    Q8RowsArgs r{};
+    r.x = x;
+    r.gamma = gamma;
+    r.eps = eps;
+    r.planes = reinterpret_cast<__nv_bfloat16*>(ctx->planes.p);
+    r.M = M;
+    r.K = K;
+    CU(launch_q8_rows(r, s));
+    return SHAINET_ATTN_OK;
+}
+
+Q8GemmOut rows_out(float* y, int N, const float* residual) { return Q8GemmOut{{y}, {0}, {N}, 1, 0, residual}; }
+
+constexpr size_t planes_floats(size_t M, size_t K) { return (3 * M * K + 1) / 2; }
+
 enum { ACT_QKV = 0, ACT_ATTN = 1, ACT_H = 2, ACT_HIDDEN = 3, ACT_A = 4, ACT_B = 5 };
+
+bool block_tensor_path(const shainet_attn_block* b) {
+    return b->qkv_maps.ok && b->wo->maps.ok && (!b->gate || (b->gate->maps.ok && b->up->maps.ok && b->down->maps.ok));
+}
+
+// Several new tokens: the projections on the tensor cores.
+int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T, cudaStream_t s) {
+    shainet_attn_ctx* ctx = b->ctx;
+    const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
+    int rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
+    if (!rc) rc = grow(ctx->act[ACT_ATTN], (size_t)T * qd, s);
+    if (!rc && b->gate) rc = grow(ctx->act[ACT_H], (size_t)T * d, s);
+    if (!rc && b->gate) rc = grow(ctx->gate_up, (size_t)T * 2 * b->ffn, s);
+    if (!rc) rc = planes_acquire(ctx, s);
+    if (!rc) rc = grow(ctx->planes, planes_floats(T, std::max(std::max(d, qd), b->ffn)), s);
+    if (rc) return rc;
+    float* qbuf = ctx->act[ACT_QKV].p;
+    float* kbuf = qbuf + (size_t)T * qd;
+    float* vbuf = kbuf + (size_t)T * kd;
+    rc = make_planes(ctx, x, T, d, b->norm1, b->eps, s);
+    if (rc) return rc;
+    const Q8GemmOut qkv{{qbuf, kbuf, vbuf}, {0, qd, qd + kd}, {qd, kd, kd}, 3, 0, nullptr};
+    rc = gemm_tc(ctx, &b->qkv_maps, nullptr, T, d, qkv, nullptr, s);
+    if (rc) return rc;
+    float* attn = ctx->act[ACT_ATTN].p;
+    rc = forward_device(ctx, b->kv, qbuf, kbuf, vbuf, attn, T, b->scale, 0, s);
+    if (!rc) rc = make_planes(ctx, attn, T, qd, nullptr, 0.0, s);
+    if (rc) return rc;
+    if (!b->gate) return gemm_tc(ctx, &b->wo->maps, nullptr, T, qd, rows_out(out, d, x), nullptr, s);
+    float* h = ctx->act[ACT_H].p;
+    int splits = 1;
+    rc = gemm_tc(ctx, &b->wo->maps, nullptr, T, qd, rows_out(h, d, x), &splits, s);
+    if (rc) return rc;
+    Q8RowsArgs r{};   // h = x + o_proj, its norm and its planes in one pass
+    r.x = splits > 1 ? ctx->gemm_part.p : h;
+    r.splits = splits > 1 ? splits : 0;
+    r.split_stride = (size_t)T * d;
+    r.residual = x;
+    r.h = h;
+    r.gamma = b->norm2;
+    r.eps = b->eps;
+    r.planes = reinterpret_cast<__nv_bfloat16*>(ctx->planes.p);
+    r.M = T;
+    r.K = d;
+    CU(launch_q8_rows(r, s));
+    rc = gemm_tc(ctx, &b->gate->maps, &b->up->maps, T, d, rows_out(ctx->gate_up.p, 2 * b->ffn, nullptr), &splits, s);
+    if (rc) return rc;
+    CU(launch_q8_swiglu(splits > 1 ? ctx->gemm_part.p : ctx->gate_up.p, splits, (size_t)T * 2 * b->ffn, T, b->ffn,
+                        reinterpret_cast<__nv_bfloat16*>(ctx->planes.p), s));
+    return gemm_tc(ctx, &b->down->maps, nullptr, T, b->ffn, rows_out(out, d, h), nullptr, s);
+}
 
 // LlamaBlock#forward_cached (llama_block.cr:189-196) on device pointers.
 int block_forward(shainet_attn_block* b, const float* x, float* out, int T, cudaStream_t s) {
+    if (T > 1 && block_tensor_path(b)) return block_forward_rows(b, x, out, T, s);
     shainet_attn_ctx* ctx = b->ctx;
     const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
     int rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
@@ -252,6 +358,7 @@ int shainet_attn_q8_create_raw(shainet_attn_ctx* ctx, shainet_attn_q8** out, con
         *out = nullptr;
         return fail_cuda(e, "upload of a Q8_0 weight");
     }
+    q8_gemm_maps(&w->maps, w->q, w->scales, N, K);
     return SHAINET_ATTN_OK;
 }
 
@@ -263,6 +370,7 @@ int shainet_attn_q8_wrap(shainet_attn_ctx* ctx, shainet_attn_q8** out, const sig
     (*out)->q = const_cast<signed char*>(q_dev);
     (*out)->scales = const_cast<float*>(scales_dev);
     (*out)->owns = false;
+    q8_gemm_maps(&(*out)->maps, q_dev, scales_dev, N, K);
     return SHAINET_ATTN_OK;
 }
 
@@ -293,6 +401,18 @@ int shainet_attn_q8_gemv_dev(shainet_attn_ctx* ctx, const shainet_attn_q8* w, co
     if (M < 0) return fail(SHAINET_ATTN_E_INVALID, "negative row count");
     DeviceGuard g(ctx->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
+    if (M > 1 && w->maps.ok && aligned16(x_dev)) {
+        int rc = planes_acquire(ctx, s);
+        if (!rc) rc = grow(ctx->planes, planes_floats(M, w->K), s);
+        if (!rc) rc = make_planes(ctx, x_dev, M, w->K, nullptr, 0.0, s);
+        if (!rc) rc = gemm_tc(ctx, &w->maps, nullptr, M, w->K, rows_out(y_dev, w->N, nullptr), nullptr, s);
+        if (rc) return rc;
+        if (!ctx->planes_ev) CU(cudaEventCreateWithFlags(&ctx->planes_ev, cudaEventDisableTiming));
+        CU(cudaEventRecord(ctx->planes_ev, s));
+        ctx->planes_stream = s;
+        ctx->planes_pending = true;
+        return SHAINET_ATTN_OK;
+    }
     return gemv(ctx, x_dev, w->q, w->scales, nullptr, nullptr, y_dev, M, w->N, w->K, nullptr, 0.0, nullptr, nullptr, nullptr, s);
 }
 
@@ -364,6 +484,7 @@ int shainet_attn_block_create(shainet_attn_ctx* ctx, shainet_attn_block** out, s
         shainet_attn_block_destroy(b);
         return fail_cuda(e, "stacking the q/k/v projections");
     }
+    q8_gemm_maps(&b->qkv_maps, b->qkv_q, b->qkv_s, (int)n_all, d_model);
     int rc = upload_vec(b->norm1, norm1_host, (size_t)d_model);
     if (!rc && has_ffn) rc = upload_vec(b->norm2, norm2_host, (size_t)d_model);
     if (rc) {
