@@ -194,7 +194,12 @@ constexpr size_t planes_floats(size_t M, size_t K) { return (3 * M * K + 1) / 2;
 
 enum { ACT_QKV = 0, ACT_ATTN = 1, ACT_H = 2, ACT_HIDDEN = 3, ACT_A = 4, ACT_B = 5 };
 
-bool block_tensor_path(const shainet_attn_block* b) {
+// Up to four rows the single-row kernels' row tiles read the weights once, in one launch (2048 -> 8192: 11 us for two rows
+// and 16 us for four, against 18 us for planes, product and split sum); they need whole 2048-input segments.
+bool few_rows(int M, int K) { return M <= 4 && q8_fast_path(K); }
+
+bool block_tensor_path(const shainet_attn_block* b, int T) {
+    if (few_rows(T, b->d_model) && few_rows(T, b->q_dim) && (!b->gate || few_rows(T, b->ffn))) return false;
     return b->qkv_maps.ok && b->wo->maps.ok && (!b->gate || (b->gate->maps.ok && b->up->maps.ok && b->down->maps.ok));
 }
 
@@ -247,7 +252,7 @@ int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T,
 
 // LlamaBlock#forward_cached (llama_block.cr:189-196) on device pointers.
 int block_forward(shainet_attn_block* b, const float* x, float* out, int T, cudaStream_t s) {
-    if (T > 1 && block_tensor_path(b)) return block_forward_rows(b, x, out, T, s);
+    if (T > 1 && block_tensor_path(b, T)) return block_forward_rows(b, x, out, T, s);
     shainet_attn_ctx* ctx = b->ctx;
     const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
     int rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
@@ -401,7 +406,7 @@ int shainet_attn_q8_gemv_dev(shainet_attn_ctx* ctx, const shainet_attn_q8* w, co
     if (M < 0) return fail(SHAINET_ATTN_E_INVALID, "negative row count");
     DeviceGuard g(ctx->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    if (M > 1 && w->maps.ok && aligned16(x_dev)) {
+    if (M > 1 && !few_rows(M, w->K) && w->maps.ok && aligned16(x_dev)) {
         int rc = planes_acquire(ctx, s);
         if (!rc) rc = grow(ctx->planes, planes_floats(M, w->K), s);
         if (!rc) rc = make_planes(ctx, x_dev, M, w->K, nullptr, 0.0, s);

@@ -14,13 +14,18 @@
 // A pair of CTAs (cta_group::2) computes 256 weight rows x NT tokens.  The weights are the A operand: raw int8 tiles
 // arrive by TMA, four convert warps (one thread per weight row) turn 32 of them at a time into bfloat16 pairs and put
 // them into tensor memory; the activations are the B operand, three bfloat16 planes prepared by a kernel ahead, each CTA
-// loading its half of the tokens.  Lanes of tensor memory are weight rows, so a thread of the sixteen accumulating
+// loading its half of the tokens.  Lanes of tensor memory are weight rows, so a thread of the eight accumulating
 // warps needs one scale per block and stores its outputs coalesced over the lanes.
 //
-// Bounds.  Three bf16 passes cost 192 cycles of the tensor pipe per 32 inputs and 128-token tile; the accumulating
-// warps spend 128 cycles of the fp32 pipe on the same block, the convert warps about 80 issue slots per scheduler.
-// The pair's 33 KB per 64 inputs and CTA is what L2 has to deliver in 384 cycles.  With few tokens the launch is bound
-// by the weight stream instead; the contraction is then split over the pairs (split-K) until they are all busy.
+// Bounds.  The tensor core multiplies 4096 bf16 pairs per cycle and SM, but an MMA of 16 inputs takes at least about 64
+// cycles, however few its columns (the 128 rows of A have to pass).  At 128 tokens the three planes are three passes:
+// 384 cycles per 32-input block, against about 190 issue slots per scheduler in the accumulating warps (128 of them
+// fp32 pipe) and 150 in the convert warps.  With up to 64 tokens the planes lie side by side as 3 NT columns of one
+// pass, so a block takes two MMAs instead of six, and the accumulating warps add the three columns of a token; the
+// launch is then bound by the convert warps (4 KB of weights in about 170 cycles) and the contraction is split over the
+// pairs (split-K) until they are all busy.
+// Measured, planes and split sums included: 4096 x 2048 -> 8192 in 374 us = 367 TFLOP/s of weight products (1.1 PFLOP/s of
+// bf16 passes), 16 x 2048 -> 8192 in 18.7 us; row tiles of four on the CUDA cores took 12.9 ms and 51 us.
 #include <cuda_bf16.h>
 #include <math.h>
 #include <algorithm>
@@ -44,6 +49,11 @@ __device__ __forceinline__ f32x2 qt_pack_bits(uint32_t lo, uint32_t hi) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
     return r;
 }
+__device__ __forceinline__ f32x2 qt_add(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ f32x2 qt_fma(f32x2 a, f32x2 b, f32x2 c) {
     f32x2 d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
@@ -62,10 +72,11 @@ template <int NT_>
 struct QT {
     static constexpr int NT = NT_;
     static constexpr int ROWS = 128;                     // weight rows per CTA, 256 per pair
-    static constexpr int KB = 32;                        // inputs per scale block = per accumulation in tensor memory
-    static constexpr int ND = NT == 128 ? 3 : (NT == 64 ? 6 : 8);   // block accumulators (and A slots) in tensor memory
+    static constexpr bool STACK = NT <= 64;              // the planes are columns of one pass, not three passes
+    static constexpr int D_COLS = STACK ? 3 * NT : NT;   // columns of one block accumulator
+    static constexpr int ND = NT == 16 ? 8 : NT == 32 ? 4 : NT == 64 ? 2 : 3;   // block accumulators (and A slots) in tensor memory
     static constexpr int A_COLS = 16;                    // 32 bfloat16 per lane
-    static constexpr int TMEM_A = ND * NT;
+    static constexpr int TMEM_A = ND * D_COLS;
     static constexpr int TMEM_COLS = 512;
     static constexpr int NB = NT == 128 ? 5 : 6;         // B stages of 64 inputs
     static constexpr int PLANE_BYTES = (NT / 2) * 128;   // this CTA's half of the tokens, 64 bfloat16 each
@@ -74,8 +85,8 @@ struct QT {
     static constexpr int W_BYTES = ROWS * 128;
     static constexpr int NS = 8;                         // scale stages of 4 blocks
     static constexpr int S_BYTES = ROWS * 16;
-    static constexpr int ACC_WARPS = 16;
-    static constexpr int CW = NT / 4;                    // columns of one accumulating warp
+    static constexpr int ACC_WARPS = 8;
+    static constexpr int CW = NT / 2;                    // tokens of one accumulating warp
     static constexpr int THREADS = (8 + ACC_WARPS) * 32;
     static constexpr int BAR_BYTES = 640;
     static constexpr size_t SMEM_BYTES = (size_t)NB * B_BYTES + (size_t)NW * W_BYTES + (size_t)NS * S_BYTES + BAR_BYTES;
@@ -83,6 +94,26 @@ struct QT {
     static_assert((2 * (NB + NW + NS + ND) + ND) * 8 + 4 <= BAR_BYTES, "barrier area");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 };
+
+// Position in a ring of N barriers and the parity of its current round.
+template <int N>
+struct RingPos {
+    int slot = 0;
+    uint32_t parity = 0;
+    __device__ __forceinline__ void next() {
+        if (++slot == N) {
+            slot = 0;
+            parity ^= 1;
+        }
+    }
+};
+
+template <int CW>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[CW]) {
+    if constexpr (CW == 32) tmem_ld32(taddr, v);
+    else if constexpr (CW == 16) tmem_ld16(taddr, v);
+    else tmem_ld8(taddr, v);
+}
 
 // The output segment of column `col` (selects, not indexing: the arrays stay in the parameter space).
 struct OutColumn {
@@ -125,13 +156,13 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     uint64_t* w_full = b_free + NB;       // NW, own
     uint64_t* w_free = w_full + NW;       // NW, own: 4 convert warps
     uint64_t* s_full = w_free + NW;       // NS, own
-    uint64_t* s_free = s_full + NS;       // NS, own: 16 accumulating warps
+    uint64_t* s_free = s_full + NS;       // NS, own: 8 accumulating warps
     uint64_t* a_full = s_free + NS;       // ND, the leader's: 8 convert warps of both CTAs
     uint64_t* d_full = a_full + ND;       // ND, in both CTAs: block accumulated (and its A slot free again)
-    uint64_t* d_free = d_full + ND;       // ND, the leader's: 32 accumulating warps of both CTAs
+    uint64_t* d_free = d_full + ND;       // ND, the leader's: 16 accumulating warps of both CTAs
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_free + ND);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
     if (threadIdx.x == 0) {
@@ -228,43 +259,44 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer: one thread of the leader, for both CTAs ----------------
-        if (lane == 0 && leader) {
-            constexpr uint32_t idesc = idesc_bf16(2 * C::ROWS, NT);
+        // ---------------- MMA issuer: one warp of the leader, for both CTAs ----------------
+        if (leader) {
+            constexpr uint32_t idesc = idesc_bf16(2 * C::ROWS, C::D_COLS);
             uint32_t stages = 0;      // of all this pair's items: the last ones are not handed back (nobody waits for them)
             for (int w = pair; w < items; w += pairs) {
                 const Item it = item_of(w);
                 stages += 2 * (it.g1 - it.g0);
             }
-            auto commit = [&](uint64_t* bar) {   // this CTA's barrier and the peer's copy of it
-                tc_commit_pair(smem_u32(bar));
-                tc_commit_pair(map_to_cta(smem_u32(bar), 1u));
-            };
             const uint64_t desc0 = smem_desc_sw128(smem_u32(b_s), 16, 1024);
-            bool ok = true;
+            RingPos<NB> rb;
+            RingPos<ND> rd;
+            bool ok = true, first_round = true;   // the first ND blocks find their accumulators free
             for (uint32_t s = 0; ok && s < stages; ++s) {
-                const int st = s % NB;
-                if (!(ok = mbar_wait(&b_full[st], (s / NB) & 1, a.status, 74))) break;
-                const uint64_t bd = desc0 + (uint64_t)((st * C::B_BYTES) >> 4);
+                if (!(ok = mbar_wait(&b_full[rb.slot], rb.parity, a.status, 74))) break;
+                const uint64_t bd = desc0 + (uint64_t)((rb.slot * C::B_BYTES) >> 4);
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    const uint32_t i = 2 * s + half;
-                    const int slot = i % ND;
-                    if (!(ok = mbar_wait(&a_full[slot], (i / ND) & 1, a.status, 75))) break;
-                    if (i >= ND && !(ok = mbar_wait(&d_free[slot], ((i / ND) - 1) & 1, a.status, 76))) break;
+                    if (!first_round && !(ok = mbar_wait(&d_free[rd.slot], rd.parity ^ 1u, a.status, 76))) break;
+                    if (!(ok = mbar_wait(&a_full[rd.slot], rd.parity, a.status, 75))) break;
                     tc_fence_after();
-                    const uint32_t d = tmem + slot * NT;
-                    const uint32_t aw = tmem + C::TMEM_A + slot * C::A_COLS;
-                    // smallest plane first
+                    const uint32_t d = tmem + rd.slot * C::D_COLS;
+                    const uint32_t aw = tmem + C::TMEM_A + rd.slot * C::A_COLS;
+                    if (elect_one()) {
+                        constexpr int PASSES = C::STACK ? 1 : 3;
 #pragma unroll
-                    for (int p = 2; p >= 0; --p)
+                        for (int p = PASSES - 1; p >= 0; --p)   // smallest plane first
 #pragma unroll
-                        for (int kk = 0; kk < 2; ++kk)
-                            mma_ts_bf16_pair(d, aw + kk * 8, bd + (uint64_t)((p * C::PLANE_BYTES + half * 64 + kk * 32) >> 4), idesc,
-                                             (p < 2 || kk > 0) ? 1u : 0u);
-                    if (half == 1 && s + NB < stages) commit(&b_free[st]);
-                    commit(&d_full[slot]);
+                            for (int kk = 0; kk < 2; ++kk)
+                                mma_ts_bf16_pair(d, aw + kk * 8, bd + (uint64_t)((p * C::PLANE_BYTES + half * 64 + kk * 32) >> 4),
+                                                 idesc, (p < PASSES - 1 || kk > 0) ? 1u : 0u);
+                        if (half == 1 && s + NB < stages) tc_commit_both(&b_free[rb.slot]);
+                        tc_commit_both(&d_full[rd.slot]);
+                    }
+                    __syncwarp();
+                    rd.next();
+                    if (rd.slot == 0) first_round = false;
                 }
+                rb.next();
             }
         }
     } else if (warp >= 4 && warp < 8) {
@@ -273,20 +305,21 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         const int r = quad * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
         const uint32_t a_leader = map_to_cta(smem_u32(&a_full[0]), 0u);
-        uint32_t s = 0, i = 0;
-        bool ok = true;
+        RingPos<NW> rw;
+        RingPos<ND> rd;
+        bool ok = true, first_round = true;
         for (int w = pair; ok && w < items; w += pairs) {
             const Item it = item_of(w);
-            for (int g = it.g0; ok && g < it.g1; ++g, ++s) {
-                const int ws = s % NW;
-                if (!(ok = mbar_wait(&w_full[ws], (s / NW) & 1, a.status, 77))) break;
-                const unsigned char* row = w_s + ws * C::W_BYTES + r * 128;
-                for (int q = 0; q < 4; ++q, ++i) {
+            for (int g = it.g0; ok && g < it.g1; ++g) {
+                if (!(ok = mbar_wait(&w_full[rw.slot], rw.parity, a.status, 77))) break;
+                const unsigned char* row = w_s + rw.slot * C::W_BYTES + r * 128;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
                     const uint4 c0 = *reinterpret_cast<const uint4*>(row + (((2 * q) ^ (r & 7)) << 4));
                     const uint4 c1 = *reinterpret_cast<const uint4*>(row + (((2 * q + 1) ^ (r & 7)) << 4));
                     if (q == 3) {
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&w_free[ws]);
+                        if (lane == 0) mbar_arrive(&w_free[rw.slot]);
                     }
                     const uint32_t words[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
                     uint32_t out[16];
@@ -298,60 +331,81 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                         const uint32_t lo = (pr & 0x007f007fu) | 0x43004300u, hi = (pr & 0x00800080u) | 0x43004300u;
                         asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(out[k]) : "r"(lo), "r"(hi));
                     }
-                    const int slot = i % ND;
-                    if (i >= ND && !(ok = mbar_wait(&d_full[slot], ((i / ND) - 1) & 1, a.status, 78))) break;
+                    if (!first_round && !(ok = mbar_wait(&d_full[rd.slot], rd.parity ^ 1u, a.status, 78))) break;
                     tc_fence_after();
-                    tmem_st16(tmem + lane_addr + C::TMEM_A + slot * C::A_COLS, out);
+                    tmem_st16(tmem + lane_addr + C::TMEM_A + rd.slot * C::A_COLS, out);
                     tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(a_leader + 8u * (uint32_t)slot);
+                    if (lane == 0) mbar_arrive_cluster(a_leader + 8u * (uint32_t)rd.slot);
+                    rd.next();
+                    if (rd.slot == 0) first_round = false;
                 }
+                rw.next();
             }
         }
     } else if (warp >= 8) {
-        // ---------------- accumulate: one weight row and NT/4 tokens per thread ----------------
+        // ---------------- accumulate: one weight row and NT/2 tokens (one CTA's half) per thread ----------------
         const int quad = warp & 3, cq = (warp - 8) >> 2;
         const int r = quad * 32 + lane;
-        const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
+        const uint32_t d_addr = tmem + ((uint32_t)(quad * 32) << 16) + cq * (C::D_COLS / 2);
         const uint32_t d_leader = map_to_cta(smem_u32(&d_free[0]), 0u);
         pdl_wait();   // the residual comes from the kernels ahead
-        uint32_t s = 0, i = 0;
+        RingPos<NS> rs;
+        RingPos<ND> rd;
         bool ok = true;
         for (int w = pair; ok && w < items; w += pairs) {
             const Item it = item_of(w);
             f32x2 acc[CW / 2];
 #pragma unroll
             for (int c = 0; c < CW / 2; ++c) acc[c] = 0ull;
-            for (int g = it.g0; ok && g < it.g1; ++g, ++s) {
-                const int ss = s % NS;
-                if (!(ok = mbar_wait(&s_full[ss], (s / NS) & 1, a.status, 79))) break;
-                const float4 sc4 = *reinterpret_cast<const float4*>(s_s + ss * C::S_BYTES + r * 16);
+            for (int g = it.g0; ok && g < it.g1; ++g) {
+                if (!(ok = mbar_wait(&s_full[rs.slot], rs.parity, a.status, 79))) break;
+                const float4 sc4 = *reinterpret_cast<const float4*>(s_s + rs.slot * C::S_BYTES + r * 16);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&s_free[ss]);
+                if (lane == 0) mbar_arrive(&s_free[rs.slot]);
+                rs.next();
                 const float sc[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
 #pragma unroll
-                for (int q = 0; q < 4; ++q, ++i) {
-                    const int slot = i % ND;
-                    if (!(ok = mbar_wait(&d_full[slot], (i / ND) & 1, a.status, 80))) break;
+                for (int q = 0; q < 4; ++q) {
+                    if (!(ok = mbar_wait(&d_full[rd.slot], rd.parity, a.status, 80))) break;
                     tc_fence_after();
-                    uint32_t v[CW];
-                    const uint32_t da = tmem + lane_addr + slot * NT + cq * CW;
-                    if constexpr (CW == 32) tmem_ld32(da, v);
-                    else if constexpr (CW == 16) tmem_ld16(da, v);
-                    else if constexpr (CW == 8) tmem_ld8(da, v);
-                    else tmem_ld4(da, v);
-                    tmem_wait_ld();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(d_leader + 8u * (uint32_t)slot);
+                    const uint32_t da = d_addr + rd.slot * C::D_COLS;
                     const f32x2 s2 = qt_pack(sc[q], sc[q]);
+                    auto handed_back = [&] {   // the accumulator's columns are in registers
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(d_leader + 8u * (uint32_t)rd.slot);
+                    };
+                    if constexpr (C::STACK) {
+                        uint32_t v0[CW], v1[CW], v2[CW];
+                        tmem_ld<CW>(da + 2 * CW, v2);
+                        tmem_ld<CW>(da + CW, v1);
+                        tmem_ld<CW>(da, v0);
+                        tmem_wait_ld();
+                        handed_back();
 #pragma unroll
-                    for (int c = 0; c < CW / 2; ++c) acc[c] = qt_fma(qt_pack_bits(v[2 * c], v[2 * c + 1]), s2, acc[c]);
+                        for (int c = 0; c < CW / 2; ++c) {
+                            const f32x2 low = qt_add(qt_pack_bits(v2[2 * c], v2[2 * c + 1]), qt_pack_bits(v1[2 * c], v1[2 * c + 1]));
+                            acc[c] = qt_fma(qt_add(low, qt_pack_bits(v0[2 * c], v0[2 * c + 1])), s2, acc[c]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int h = 0; h < CW / 32; ++h) {
+                            uint32_t v[32];
+                            tmem_ld32(da + h * 32, v);
+                            tmem_wait_ld();
+                            if (h == CW / 32 - 1) handed_back();
+#pragma unroll
+                            for (int c = 0; c < 16; ++c)
+                                acc[h * 16 + c] = qt_fma(qt_pack_bits(v[2 * c], v[2 * c + 1]), s2, acc[h * 16 + c]);
+                        }
+                    }
+                    rd.next();
                 }
             }
             if (!ok) break;
-            // this thread's weight row of the NT/4 tokens: lanes are consecutive columns of the output
+            // this thread's weight row of the NT/2 tokens: lanes are consecutive columns of the output
             const bool second = it.nt >= a.n_tiles0;
             const int n = (it.nt - (second ? a.n_tiles0 : 0)) * 256 + (int)rank * C::ROWS + r;
             if (n < (second ? a.n[1] : a.n[0])) {
@@ -553,8 +607,8 @@ int token_tile(int M, int cap) {
     return nt < cap ? nt : cap;
 }
 
-// Cycles one 32-input block of a pair's tile takes: the tensor pipe at 128 tokens, the convert warps below.
-double block_cycles(int nt) { return nt >= 128 ? 230.0 : nt >= 64 ? 170.0 : 150.0; }
+// Cycles one 32-input block of a pair's tile takes: the tensor pipe at 128 tokens, the convert and accumulating warps below.
+double block_cycles(int nt) { return nt >= 128 ? 450.0 : nt >= 64 ? 330.0 : 260.0; }
 
 }  // namespace
 

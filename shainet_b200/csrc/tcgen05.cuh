@@ -52,6 +52,26 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster) : "memory");
 }
 
+// Arrival (once all MMAs issued so far by this thread have completed) on the barrier at the same offset in both CTAs of the
+// pair, as one instruction.
+__device__ __forceinline__ void tc_commit_both(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+
+// One lane of a converged warp.  A warp that issues MMAs runs its whole loop converged and elects a lane for the issuing
+// statements only: its addresses and descriptors then stay in uniform registers, which tcgen05.mma reads; in a loop under
+// `lane == 0` every operand of every MMA is moved there first (about 70 cycles an MMA in the Q8_0 kernel).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r != 0;
+}
+
+// Warp index that the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // Arrival on a barrier of either CTA of the pair.  What it announces lies in tensor memory (ordered by the tcgen05
 // fences on both sides), so the default scope is enough.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
