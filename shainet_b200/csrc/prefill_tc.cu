@@ -119,7 +119,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     uint64_t* o_done = p_full + 4;      // [tile] = 2
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     // the two tiles of this CTA; heaviest (latest rows) first
     const int x = gridDim.x - 1 - blockIdx.x;
     int th[2], ti0[2], trows[2], tn[2];
@@ -196,8 +196,8 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // ---------------- MMA issuer: a converged warp (see elect_one) ----------------
+        {
             constexpr uint32_t idesc_qk = idesc_tf32(C::BM, C::BN, 0, 0);
             constexpr uint32_t idesc_pv = idesc_tf32(C::BM, HD, 0, 1);
             const uint32_t q_addr = smem_u32(q_s), k_addr0 = smem_u32(k_s), v_addr = smem_u32(v_s);
@@ -207,15 +207,21 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 for (int t = 0; t < 2; ++t) {
                     if (j >= tn[t]) continue;
                     const uint32_t d = tmem + C::TMEM_S + (t * 2 + (j & 1)) * C::BN;
+                    const uint64_t q_desc0 = smem_desc_sw128(q_addr + t * C::Q_BYTES, 16, 1024);
+                    const uint64_t k_desc0 = smem_desc_sw128(k_addr, 16, 1024);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < HD / 8; ++kk) {
-                        const uint64_t ad = smem_desc_sw128(q_addr + t * C::Q_BYTES + (kk >> 2) * (C::BM * 128) + (kk & 3) * 32, 16, 1024);
-                        const uint64_t bd = smem_desc_sw128(k_addr + (kk >> 2) * (C::BN * 128) + (kk & 3) * 32, 16, 1024);
-                        mma_ss_tf32(d, ad, bd, idesc_qk, kk > 0);
+                        for (int kk = 0; kk < HD / 8; ++kk) {
+                            const uint64_t ad = q_desc0 + (uint64_t)(((kk >> 2) * (C::BM * 128) + (kk & 3) * 32) >> 4);
+                            const uint64_t bd = k_desc0 + (uint64_t)(((kk >> 2) * (C::BN * 128) + (kk & 3) * 32) >> 4);
+                            mma_ss_tf32(d, ad, bd, idesc_qk, kk > 0);
+                        }
+                        tc_commit(&s_full[t * 2 + (j & 1)]);
                     }
-                    tc_commit(&s_full[t * 2 + (j & 1)]);
+                    __syncwarp();
                 }
-                tc_commit(&k_empty[j & 1]);
+                if (elect_one()) tc_commit(&k_empty[j & 1]);
+                __syncwarp();
             };
             bool ok = n > 0 && mbar_wait(q_full, 0, a.status, 33);
             if (ok && (ok = mbar_wait(&k_full[0], 0, a.status, 34))) {
@@ -237,15 +243,18 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     tc_fence_after();
                     const uint32_t d = tmem + C::TMEM_O + t * HD;
                     const uint32_t p = tmem + C::TMEM_S + (t * 2 + b) * C::BN;
+                    const uint64_t v_desc0 = smem_desc(v_addr, C::BN * 128, 512, LAYOUT_SW128_BASE32B);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < C::BN / 8; ++kk) {
-                        const uint64_t bd = smem_desc(v_addr + kk * 1024, C::BN * 128, 512, LAYOUT_SW128_BASE32B);
-                        mma_ts_tf32(d, p + kk * 8, bd, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                        for (int kk = 0; kk < C::BN / 8; ++kk)
+                            mma_ts_tf32(d, p + kk * 8, v_desc0 + (uint64_t)(kk * 1024 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                        tc_commit(&o_done[t]);
                     }
-                    tc_commit(&o_done[t]);
+                    __syncwarp();
                 }
                 if (!ok) break;
-                tc_commit(v_empty);
+                if (elect_one()) tc_commit(v_empty);
+                __syncwarp();
             }
         }
     } else if (warp >= 4) {
@@ -415,7 +424,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     static_assert((1 + 2 * KS + 2 * VS + 2 * SB + 1 + 4) * 8 + 4 <= C::BAR_BYTES, "barrier area");
     static_assert(C::TMEM_O + HD <= C::TMEM_COLS, "tensor memory columns");
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
     // heaviest (latest rows) first
@@ -488,30 +497,28 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer: one thread of the leader, for both CTAs ----------------
-        if (lane == 0 && leader && n > 0) {
+        // ---------------- MMA issuer: one warp of the leader, for both CTAs (see elect_one) ----------------
+        if (leader && n > 0) {
             constexpr uint32_t idesc_qk = idesc_tf32(2 * C::BM, C::BN, 0, 0);
             constexpr uint32_t idesc_pv = idesc_tf32(2 * C::BM, HD, 0, 1);
             const uint32_t q_addr = smem_u32(q_s), k_addr0 = smem_u32(k_s), v_addr0 = smem_u32(v_s);
-            auto commit = [&](uint64_t* bar) {   // this CTA's barrier and the peer's copy of it
-                tc_commit_pair(smem_u32(bar));
-                tc_commit_pair(map_to_cta(smem_u32(bar), 1u));
-            };
             // A descriptor differs from the one of the tile's first bytes only in its address field (bits 0-13, in
-            // units of 16 bytes; every address here is below 256 KB): built once, then one 64-bit add per MMA by this
-            // single issuing thread.
+            // units of 16 bytes; every address here is below 256 KB): built once, then one 64-bit add per MMA.
             const uint64_t q_desc0 = smem_desc_sw128(q_addr, 16, 1024);
             auto scores = [&](int j) {
                 const uint64_t k_desc0 = smem_desc_sw128(k_addr0 + (j % KS) * C::K_BYTES, 16, 1024);
                 const uint32_t d = tmem + C::TMEM_S + (j % SB) * C::BN;
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < HD / 8; ++kk) {
-                    const uint64_t ad = q_desc0 + (uint64_t)(((kk >> 2) * (C::BM * 128) + (kk & 3) * 32) >> 4);
-                    const uint64_t bd = k_desc0 + (uint64_t)(((kk >> 2) * (C::K_ROWS * 128) + (kk & 3) * 32) >> 4);
-                    mma_ss_tf32_pair(d, ad, bd, idesc_qk, kk > 0);
+                    for (int kk = 0; kk < HD / 8; ++kk) {
+                        const uint64_t ad = q_desc0 + (uint64_t)(((kk >> 2) * (C::BM * 128) + (kk & 3) * 32) >> 4);
+                        const uint64_t bd = k_desc0 + (uint64_t)(((kk >> 2) * (C::K_ROWS * 128) + (kk & 3) * 32) >> 4);
+                        mma_ss_tf32_pair(d, ad, bd, idesc_qk, kk > 0);
+                    }
+                    tc_commit_both(&s_full[j % SB]);
+                    tc_commit_both(&k_empty[j % KS]);
                 }
-                commit(&s_full[j % SB]);
-                commit(&k_empty[j % KS]);
+                __syncwarp();
             };
             // scores run SB - 1 steps ahead of P.V
             bool ok = mbar_wait(q_full, 0, a.status, 53);
@@ -534,11 +541,14 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
                 const uint32_t d = tmem + C::TMEM_O;
                 const uint32_t p = tmem + C::TMEM_S + (j % SB) * C::BN;
                 const uint64_t v_desc0 = smem_desc(v_addr0 + sv * C::V_BYTES, C::BN * 128, 512, LAYOUT_SW128_BASE32B);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < C::BN / 8; ++kk)
-                    mma_ts_tf32_pair(d, p + kk * 8, v_desc0 + (uint64_t)(kk * 1024 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-                commit(o_done);
-                commit(&v_empty[sv]);
+                    for (int kk = 0; kk < C::BN / 8; ++kk)
+                        mma_ts_tf32_pair(d, p + kk * 8, v_desc0 + (uint64_t)(kk * 1024 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                    tc_commit_both(o_done);
+                    tc_commit_both(&v_empty[sv]);
+                }
+                __syncwarp();
             }
         }
     } else if (warp >= 4) {

@@ -46,12 +46,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
         : "memory");
 }
 
-// Arrival (once all MMAs issued so far by this thread have completed) on a barrier given by its
-// shared::cluster address: the local one or the peer's copy.
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster) : "memory");
-}
-
 // Arrival (once all MMAs issued so far by this thread have completed) on the barrier at the same offset in both CTAs of the
 // pair, as one instruction.
 __device__ __forceinline__ void tc_commit_both(uint64_t* bar) {
