@@ -22,7 +22,7 @@ namespace {
 thread_local std::string g_last_error;
 
 constexpr size_t SMALL_COPY = 1 << 20;  // host entry: stage through pinned memory below this
-constexpr int SPLITK_MAX_T = 16;      // rows per call the decode kernel takes before the generic one
+constexpr int SPLITK_MAX_T = 16;      // new tokens per call the plain split-K kernel takes (forced, or behind the reference's symbol)
 constexpr int TENSOR_MIN_T = 64;      // rows per call from which the tensor-core prefill kernel takes over
 
 }  // namespace
@@ -198,7 +198,7 @@ int check_status(shainet_attn_ctx* ctx) {
     return SHAINET_ATTN_OK;
 }
 
-enum class Kernel { Generic, SplitK, Tensor };
+enum class Kernel { Generic, SplitK, Rows, Tensor };
 
 int ensure_tickets(shainet_attn_ctx* ctx, size_t n, cudaStream_t s) {
     if (ctx->tickets_cap >= n && ctx->tickets) return SHAINET_ATTN_OK;
@@ -232,7 +232,9 @@ int pick_kernel(const HeadShape& hs, int batch, int T, unsigned flags, Kernel* o
         *out = Kernel::Generic;
         return SHAINET_ATTN_OK;
     }
-    *out = (sk_ok && T <= SPLITK_MAX_T) ? Kernel::SplitK : (tc_ok && T >= TENSOR_MIN_T) ? Kernel::Tensor : Kernel::Generic;
+    if ((flags & SHAINET_ATTN_F_UNFUSED) && sk_ok && T <= SPLITK_MAX_T) *out = Kernel::SplitK;
+    else if (tc_ok && T >= TENSOR_MIN_T) *out = Kernel::Tensor;
+    else *out = attn_rows_supported(hs) && (long long)batch * T <= 65535 ? Kernel::Rows : Kernel::Generic;
     return SHAINET_ATTN_OK;
 }
 
@@ -251,14 +253,14 @@ void plan_splits(int sm_count, const HeadShape& hs, int rows, long long total_vi
     (void)rows;
 }
 
-int run_attention_untimed(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int batch, int T,
+int run_attention_untimed(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int kv_elem_bytes, int batch, int T,
                           long long total_visible, int max_visible, const float* q_rot, float* out, float scale,
                           unsigned flags, cudaStream_t s);
 
-int run_attention(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int batch, int T, long long total_visible,
+int run_attention(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int kv_elem_bytes, int batch, int T, long long total_visible,
                   int max_visible, const float* q_rot, float* out, float scale, unsigned flags, cudaStream_t s) {
     if (!ctx->timing)
-        return run_attention_untimed(ctx, hs, seqs, batch, T, total_visible, max_visible, q_rot, out, scale, flags, s);
+        return run_attention_untimed(ctx, hs, seqs, kv_elem_bytes, batch, T, total_visible, max_visible, q_rot, out, scale, flags, s);
     std::pair<cudaEvent_t, cudaEvent_t> ev;
     if (!ctx->ev_pool.empty()) {
         ev = ctx->ev_pool.back();
@@ -268,13 +270,13 @@ int run_attention(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int b
         CU(cudaEventCreate(&ev.second));
     }
     CU(cudaEventRecord(ev.first, s));
-    int rc = run_attention_untimed(ctx, hs, seqs, batch, T, total_visible, max_visible, q_rot, out, scale, flags, s);
+    int rc = run_attention_untimed(ctx, hs, seqs, kv_elem_bytes, batch, T, total_visible, max_visible, q_rot, out, scale, flags, s);
     CU(cudaEventRecord(ev.second, s));
     ctx->timed.push_back(ev);
     return rc;
 }
 
-int run_attention_untimed(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int batch, int T,
+int run_attention_untimed(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int kv_elem_bytes, int batch, int T,
                           long long total_visible, int max_visible, const float* q_rot, float* out, float scale,
                           unsigned flags, cudaStream_t s) {
     Kernel kern;
@@ -300,6 +302,19 @@ int run_attention_untimed(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seq
         return SHAINET_ATTN_OK;
     }
     const int rows = batch * T;
+    if (kern == Kernel::Rows) {
+        const AttnRowsPlan p = attn_rows_plan(hs, batch, T, total_visible, max_visible, kv_elem_bytes, ctx->sm_count);
+        a.chunk_rows = p.chunk_rows;
+        a.max_splits = p.max_splits;
+        if (a.max_splits > 1) {
+            rc = grow(ctx->part, splitk_scratch_floats(hs, rows, a.max_splits), s);
+            if (rc) return rc;
+            a.part_o = ctx->part.p;
+            a.part_ml = ctx->part.p + (size_t)rows * hs.num_heads * a.max_splits * hs.head_dim;
+        }
+        CU(launch_attn_rows(a, p.bm, kv_elem_bytes, s));
+        return SHAINET_ATTN_OK;
+    }
     plan_splits(ctx->sm_count, hs, rows, total_visible, max_visible, batch > 1 ? 8 : 1, &a.chunk_rows, &a.max_splits);
     if (a.max_splits > 1) {
         const size_t need = splitk_scratch_floats(hs, rows, a.max_splits);
@@ -322,13 +337,21 @@ int validate_forward(shainet_attn_ctx* ctx, shainet_attn_kv* kv, const void* q, 
     return SHAINET_ATTN_OK;
 }
 
+// Sixteen query heads per kv head: the fused decode kernel keeps q and the output of a group in registers and spills
+// there (28 us for a 44-row context, 66 us for 31k bfloat16 rows of a 32/2-head shape); the row-tile kernel takes the
+// group as one 16-row tile.  Only the fused kernel serves parts of a sequence, peers and log-sum-exp outputs.
+bool single_token_rows(const shainet_attn_ctx* ctx, const HeadShape& hs, unsigned flags, int pos_delta, int no_append) {
+    return hs.num_heads / hs.num_kv_heads == 16 && pos_delta == 0 && !no_append && !ctx->gather_armed && ctx->lse_out == nullptr &&
+           !(flags & (SHAINET_ATTN_F_SPLITK | SHAINET_ATTN_F_TICKET_MERGE));
+}
+
 // One call = `batch` sequences x T new tokens: norm/RoPE/append + attention.
 // `par` supplies the shared head shape, RoPE table, norm weights and biases.
 int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int batch, int T, long long total_visible,
              int max_visible, const float* q, const float* k_new, const float* v_new, float* out, float scale,
              unsigned flags, cudaStream_t s, int pos_delta = 0, int no_append = 0) {
     const HeadShape hs = par->hs;
-    const bool fused = T == 1 && splitk_supported(hs) &&
+    const bool fused = T == 1 && splitk_supported(hs) && !single_token_rows(ctx, hs, flags, pos_delta, no_append) &&
                        !(flags & (SHAINET_ATTN_F_GENERIC | SHAINET_ATTN_F_UNFUSED | SHAINET_ATTN_F_TENSOR));
     int rc;
     if (!fused && (pos_delta != 0 || no_append))
@@ -337,8 +360,13 @@ int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int
         ctx->gather_armed = false;
         return fail(SHAINET_ATTN_E_UNSUPPORTED, "peer delivery is done by the fused decode kernel only (one new token, head_dim 64/128)");
     }
-    if (!fused && par->es != 4 && seqs.many != nullptr)
-        return fail(SHAINET_ATTN_E_UNSUPPORTED, "batched decode over bfloat16 caches is served by the fused decode kernel only");
+    Kernel kern = Kernel::SplitK;
+    if (!fused) {
+        rc = pick_kernel(hs, batch, T, flags, &kern);
+        if (rc) return rc;
+    }
+    if (!fused && kern != Kernel::Rows && par->es != 4 && seqs.many != nullptr)
+        return fail(SHAINET_ATTN_E_UNSUPPORTED, "batched decode over bfloat16 caches is not served by a forced kernel");
     if (!fused) {
         ctx->last_fused = false;
         rc = grow(ctx->q_rot, (size_t)batch * T * hs.num_heads * hs.head_dim, s);
@@ -359,14 +387,11 @@ int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int
         p.batch = batch;
         p.T = T;
         p.hs = hs;
-        Kernel kern;
-        rc = pick_kernel(hs, batch, T, flags, &kern);
-        if (rc) return rc;
         p.round_q_tf32 = kern == Kernel::Tensor ? 1 : 0;
         p.kv_elem_bytes = par->es;
         p.status = ctx->status_dev;
         CU(launch_prep_append(p, s));
-        if (par->es != 4) {
+        if (par->es != 4 && kern != Kernel::Rows) {
             // These attention kernels read fp32 rows.  A bfloat16 cache is widened (exactly) into
             // a scratch image first; the capacity of the image is a whole number of the
             // tensor-core kernel's 128-row tiles, and it never holds anything but finite values.
@@ -382,7 +407,7 @@ int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int
             CU(launch_kv_convert(seqs.one.v, par->es, seqs.one.capacity, wv, 4, cap_s, hs.num_kv_heads, hs.head_dim, 0, max_visible, s));
             seqs.one = SeqDesc{wk, wv, seqs.one.start, cap_s};
         }
-        return run_attention(ctx, hs, seqs, batch, T, total_visible, max_visible, ctx->q_rot.p, out, scale, flags, s);
+        return run_attention(ctx, hs, seqs, par->es, batch, T, total_visible, max_visible, ctx->q_rot.p, out, scale, flags, s);
     }
     FusedArgs f{};
     f.q = q;

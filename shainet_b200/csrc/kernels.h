@@ -139,6 +139,17 @@ cudaError_t launch_attn_splitk(const AttnArgs& a, cudaStream_t s);
 // programmatic stream serialization.
 cudaError_t launch_decode_fused(const FusedArgs& a, cudaStream_t s);
 
+// fp32 attention of a few query rows (any group size, head_dim 64 or 128): 2..63 new tokens, or single tokens of group
+// sizes the fused decode kernel has no instance for.  chunk_rows and max_splits of the arguments come from the plan.
+struct AttnRowsPlan {
+    int bm;           // query rows (token, head of the group) per CTA
+    int chunk_rows;   // cache rows per split
+    int max_splits;
+};
+bool attn_rows_supported(const HeadShape& hs);
+AttnRowsPlan attn_rows_plan(const HeadShape& hs, int batch, int T, long long total_visible, int max_visible, int kv_elem_bytes, int sm_count);
+cudaError_t launch_attn_rows(const AttnArgs& a, int bm, int kv_elem_bytes, cudaStream_t s);
+
 // Causal prefill on the tcgen05 tensor cores (TF32): head_dim 64 or 128, one
 // sequence, q already rotated, cache already appended.  Rows of the cache
 // beyond the appended length must hold finite values (the caches are zeroed

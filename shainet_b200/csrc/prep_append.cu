@@ -23,6 +23,13 @@ namespace {
 constexpr int PREP_WARPS = 4;
 constexpr int PREP_THREADS = PREP_WARPS * 32;
 
+// The kernel ahead in the stream is complete once the wait returns (q, k and v may be its output); the kernel behind may
+// become resident from then on and does its own waiting.
+__device__ __forceinline__ void chain_wait_and_release() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // One CTA per new token.  All of the token's q, k and v heads are staged in
 // shared memory (rows padded by one float), so that
 //   * cos/sin of the token's position are computed once and shared by every head,
@@ -52,6 +59,7 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_append_kernel(PrepArgs a) {
     const SeqDesc sd = a.seqs.many ? a.seqs.many[b] : a.seqs.one;
     const int pos = sd.start + t;
     const float fpos = (float)pos;
+    chain_wait_and_release();
 
     for (int i = threadIdx.x; i < half; i += PREP_THREADS) {
         const float angle = __fmul_rn(fpos, a.inv_freq[i]);
@@ -198,6 +206,7 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_append_hd_kernel(PrepArgs a
         fence_mbar_init();
     }
     __syncthreads();
+    chain_wait_and_release();
     if (threadIdx.x == 0) {
         mbar_arrive_expect_tx(bar, (uint32_t)per_row * HD * 4);
         for (int slot = 0; slot < per_row; ++slot) {
@@ -419,10 +428,19 @@ cudaError_t launch_prep_append(const PrepArgs& a, cudaStream_t s) {
         if (e != cudaSuccess) return e;
     }
     const bool aligned = ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_new) | reinterpret_cast<uintptr_t>(a.v_new)) & 15u) == 0;
-    if (aligned && smem <= 48 * 1024 && a.hs.head_dim == 128) prep_append_hd_kernel<128><<<(unsigned)rows, PREP_THREADS, smem, s>>>(a);
-    else if (aligned && smem <= 48 * 1024 && a.hs.head_dim == 64) prep_append_hd_kernel<64><<<(unsigned)rows, PREP_THREADS, smem, s>>>(a);
-    else prep_append_kernel<<<(unsigned)rows, PREP_THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)rows);
+    cfg.blockDim = dim3(PREP_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (aligned && smem <= 48 * 1024 && a.hs.head_dim == 128) return cudaLaunchKernelEx(&cfg, prep_append_hd_kernel<128>, a);
+    if (aligned && smem <= 48 * 1024 && a.hs.head_dim == 64) return cudaLaunchKernelEx(&cfg, prep_append_hd_kernel<64>, a);
+    return cudaLaunchKernelEx(&cfg, prep_append_kernel, a);
 }
 
 cudaError_t launch_ref_append(const float* staging, float* kc, float* vc, int new_tokens, int start_pos,
