@@ -140,3 +140,25 @@ def test_cluster_pair_kernel_group_sizes_and_ragged_edges(ctx, H, KV, hd, T, pre
     per_row = np.abs(got - ref).max(axis=1) / np.abs(ref).max(axis=1)
     assert per_row.max() <= 4 * PREFILL_TOL, (float(per_row.max()), int(per_row.argmax()))
     g.close()
+
+
+@pytest.mark.parametrize("G,T,pre", [(2, 64, 0), (4, 130, 77), (8, 385, 0), (16, 127, 300)], ids=lambda v: str(v))
+def test_pair_of_ctas_at_head_dim_64(ctx, G, T, pre):
+    """What the library chooses by itself at head_dim 64 with an even group size (the pair of CTAs), over row and position
+    tiles with remainders; a call that forces the tensor kernel runs the one-CTA kernel there."""
+    import shainet_b200 as S
+    shape = dict(H=2 * G, KV=2, hd=64, theta=10000.0)
+    rng = np.random.default_rng(64 + G)
+    o, g = make_pair(ctx, shape, rng)
+    _, g1 = make_pair(ctx, shape, rng)
+    for n, flags in ((pre, S.F_GENERIC), (T, 0)):
+        if n == 0:
+            continue
+        q, k, v = qkv(rng, shape, n)
+        ref = o.attend_cached(q, k, v, threads=8)
+        got = g.forward_cached(q, k, v, flags)
+        one = g1.forward_cached(q, k, v, flags or S.F_TENSOR)
+    assert rel_err(got, ref) <= PREFILL_TOL, rel_err(got, ref)
+    assert rel_err(one, ref) <= PREFILL_TOL, rel_err(one, ref)
+    assert not np.array_equal(got, one)
+    g.close(); g1.close()
