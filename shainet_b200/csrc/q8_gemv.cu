@@ -89,17 +89,23 @@ __device__ __forceinline__ unsigned float_key(float v) {
 // chunk is at chunk*512 + j*128 + l*4 and a warp's 128-bit loads touch 512 consecutive bytes.
 // Each thread owns up to Q8_XREG float4 of a row (destination order); the norm weights for
 // them are constants and are fetched before the wait for the previous kernel.
+// Rows are padded with zeros to a whole number of chunks in shared memory; the last segment of a row may be short.  K is any
+// multiple of 128: what the bulk copies need for 16-byte pieces of the scales.  (Widths that are no multiple of 2048 went
+// through the scalar kernel below: eight greedy tokens of a 4-layer model of width 1536, FFN 4608, vocabulary 50257 took
+// 3138 us, now 1212 us.)
+__host__ __device__ constexpr int padded_k(int K) { return (K + Q8_CHUNK - 1) / Q8_CHUNK * Q8_CHUNK; }
+__host__ __device__ constexpr int segments(int K) { return (K + Q8_SEG - 1) / Q8_SEG; }
+
 constexpr int Q8_XREG = 4;   // covers K <= 4096 from registers; wider rows re-read x from L2
 
 template <int MB>
 __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows, float* xs, double* red,
                                            const float4 (&gam)[Q8_XREG]) {
-    const int K = a.K;
-    const int n4 = K >> 2;
-    const bool in_regs = n4 <= Q8_XREG * Q8_THREADS;
+    const int n4 = a.K >> 2, K = padded_k(a.K), d4 = K >> 2;   // float4 of a row, and of its image in shared memory
+    const bool in_regs = d4 <= Q8_XREG * Q8_THREADS;
     for (int m = 0; m < MB; ++m) {
         const bool live = m < rows;
-        const float4* src = reinterpret_cast<const float4*>(a.x + (size_t)(m0 + (live ? m : 0)) * K);
+        const float4* src = reinterpret_cast<const float4*>(a.x + (size_t)(m0 + (live ? m : 0)) * a.K);
         float4* dst = reinterpret_cast<float4*>(xs + (size_t)m * K);
         // destination float4 d = chunk*128 + j*32 + l  <-  source float4 chunk*128 + l*4 + j
         auto source_of = [](int d) { return ((d >> 7) << 7) + ((d & 31) << 2) + ((d >> 5) & 3); };
@@ -108,18 +114,18 @@ __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows
 #pragma unroll
         for (int it = 0; it < Q8_XREG; ++it) {
             const int d = threadIdx.x + it * Q8_THREADS;
-            xr[it] = (live && d < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xr[it] = (live && source_of(d) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (a.gamma == nullptr) {
             if (in_regs) {
 #pragma unroll
                 for (int it = 0; it < Q8_XREG; ++it) {
                     const int d = threadIdx.x + it * Q8_THREADS;
-                    if (d < n4) dst[d] = xr[it];
+                    if (d < d4) dst[d] = xr[it];
                 }
             } else {
-                for (int d = threadIdx.x; d < n4; d += Q8_THREADS)
-                    dst[d] = live ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int d = threadIdx.x; d < d4; d += Q8_THREADS)
+                    dst[d] = (live && source_of(d) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             continue;
         }
@@ -144,7 +150,7 @@ __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows
 #pragma unroll
         for (int w = 0; w < Q8_WARPS; ++w) tot += red[w];
         // 1 / rms; rsqrt is within an ulp of the f64 quotient, far below the fp32 rounding that follows
-        const double inv_rms = rsqrt(tot / (double)K + a.eps);
+        const double inv_rms = rsqrt(tot / (double)a.K + a.eps);
         // rms_norm.cr:32: f32((f64 x / rms) * f64 g), the division as a product with 1/rms
         auto normed = [&](float4 v, float4 g) {
             v.x = (float)(((double)v.x * inv_rms) * (double)g.x);
@@ -157,13 +163,13 @@ __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows
 #pragma unroll
             for (int it = 0; it < Q8_XREG; ++it) {
                 const int d = threadIdx.x + it * Q8_THREADS;
-                if (d < n4) dst[d] = normed(xr[it], gam[it]);
+                if (d < d4) dst[d] = normed(xr[it], gam[it]);
             }
         } else {
-            for (int d = threadIdx.x; d < n4; d += Q8_THREADS) {
+            for (int d = threadIdx.x; d < d4; d += Q8_THREADS) {
                 const int s = source_of(d);
-                const float4 v = live ? __ldcg(src + s) : make_float4(0.f, 0.f, 0.f, 0.f);
-                dst[d] = normed(v, __ldg(reinterpret_cast<const float4*>(a.gamma) + s));
+                const float4 v = (live && s < n4) ? __ldcg(src + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+                dst[d] = s < n4 ? normed(v, __ldg(reinterpret_cast<const float4*>(a.gamma) + s)) : v;
             }
         }
     }
@@ -188,8 +194,9 @@ __device__ __forceinline__ void load_unit(const Q8GemvArgs& a, int pair, int seg
         const float* srow = sbase + (size_t)(valid ? n : 0) * kb + seg * (Q8_SEG / 32) + (lane >> 1);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            u.w[c][j] = valid ? ldg_stream_v4(qrow + j * Q8_CHUNK) : make_uint4(0u, 0u, 0u, 0u);
-            u.s[c][j] = valid ? __ldg(srow + j * (Q8_CHUNK / 32)) : 0.0f;
+            const bool in = valid && seg * Q8_SEG + j * Q8_CHUNK + lane * 16 < a.K;   // past the end: zero scales (and x)
+            u.w[c][j] = in ? ldg_stream_v4(qrow + j * Q8_CHUNK) : make_uint4(0u, 0u, 0u, 0u);
+            u.s[c][j] = in ? __ldg(srow + j * (Q8_CHUNK / 32)) : 0.0f;
         }
     }
 }
@@ -198,6 +205,7 @@ template <int MB>
 __device__ __forceinline__ void consume_unit(const Unit& u, const float* xs, int K, int seg, int lane, float (&acc)[MB][2]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
+        if ((seg * 4 + j) * Q8_CHUNK >= K) break;   // K: the padded row length
         float4 xv[MB][4];
 #pragma unroll
         for (int m = 0; m < MB; ++m)
@@ -238,7 +246,7 @@ __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * MB;
     const int rows = min(MB, a.M - m0);
-    const int nseg = a.K / Q8_SEG;
+    const int nseg = segments(a.K);
     const int pairs = SWIGLU ? a.N : (a.N + 1) / 2;
     const int gw = blockIdx.x * Q8_WARPS + warp, tw = gridDim.x * Q8_WARPS;
 
@@ -249,8 +257,9 @@ __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8
 #pragma unroll
     for (int it = 0; it < Q8_XREG; ++it) {
         const int d = threadIdx.x + it * Q8_THREADS;
-        gam[it] = (a.gamma != nullptr && d < (a.K >> 2) && (a.K >> 2) <= Q8_XREG * Q8_THREADS)
-                      ? __ldg(reinterpret_cast<const float4*>(a.gamma) + ((d >> 7) << 7) + ((d & 31) << 2) + ((d >> 5) & 3))
+        const int src = ((d >> 7) << 7) + ((d & 31) << 2) + ((d >> 5) & 3);
+        gam[it] = (a.gamma != nullptr && src < (a.K >> 2) && padded_k(a.K) <= 4 * Q8_XREG * Q8_THREADS)
+                      ? __ldg(reinterpret_cast<const float4*>(a.gamma) + src)
                       : make_float4(1.f, 1.f, 1.f, 1.f);
     }
     // Dependents are released only after this kernel's own wait has returned: at most one
@@ -276,7 +285,7 @@ __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8
             const int npair = more_seg ? pair : pair + tw;
             const bool have_next = npair < pairs;
             if (have_next) load_unit<SWIGLU>(a, npair, more_seg ? seg + 1 : 0, lane, nxt);
-            consume_unit<MB>(cur, q8_xs, a.K, seg, lane, acc);
+            consume_unit<MB>(cur, q8_xs, padded_k(a.K), seg, lane, acc);
             if (have_next) cur = nxt;
         }
 #pragma unroll
@@ -367,10 +376,11 @@ template <int NS, bool SWIGLU>
 __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs a, int quads_per_cta) {
     extern __shared__ __align__(128) unsigned char rg_raw[];
     unsigned char* ring = rg_raw;                                             // [NS][RG_STAGE]
-    float* xs = reinterpret_cast<float*>(rg_raw + (size_t)NS * RG_STAGE);     // [K] permuted activations
-    const int nseg = a.K / Q8_SEG;
+    const int Kp = padded_k(a.K);
+    float* xs = reinterpret_cast<float*>(rg_raw + (size_t)NS * RG_STAGE);     // [Kp] permuted activations
+    const int nseg = segments(a.K);
     const int vmul = SWIGLU ? 2 : 1;
-    float* part = xs + a.K;                                                   // [local stages][RG_COLS]
+    float* part = xs + Kp;                                                   // [local stages][RG_COLS]
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(part + (size_t)quads_per_cta * vmul * nseg * RG_COLS);
     uint64_t* empty_bar = full_bar + NS;
     double* red = reinterpret_cast<double*>(empty_bar + NS);                  // [RG_NW]
@@ -399,11 +409,12 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
         const signed char* qb = (second ? a.q2 : a.q) + (size_t)quad * RG_COLS * a.K + (size_t)seg * Q8_SEG;
         const float* sb = (second ? a.scales2 : a.scales) + (size_t)quad * RG_COLS * (a.K >> 5) + seg * (Q8_SEG / 32);
         unsigned char* st = ring + (size_t)slot * RG_STAGE;
-        mbar_arrive_expect_tx(&full_bar[slot], RG_STAGE);
+        const uint32_t n = min(Q8_SEG, a.K - seg * Q8_SEG);   // the last segment of a row may be short
+        mbar_arrive_expect_tx(&full_bar[slot], RG_COLS * (n + n / 8));
 #pragma unroll
         for (int c = 0; c < RG_COLS; ++c) {
-            bulk_g2s(st + c * Q8_SEG, qb + (size_t)c * a.K, Q8_SEG, &full_bar[slot]);
-            bulk_g2s(st + RG_WBYTES + c * (Q8_SEG / 8), sb + (size_t)c * (a.K >> 5), Q8_SEG / 8, &full_bar[slot]);
+            bulk_g2s(st + c * Q8_SEG, qb + (size_t)c * a.K, n, &full_bar[slot]);
+            bulk_g2s(st + RG_WBYTES + c * (Q8_SEG / 8), sb + (size_t)c * (a.K >> 5), n / 8, &full_bar[slot]);
         }
     };
 
@@ -417,14 +428,14 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
         }
     } else {
         // ---------------- consumers ----------------
-        const int n4 = a.K >> 2;
+        const int n4 = a.K >> 2, d4 = Kp >> 2;
         auto source_of = [](int d) { return ((d >> 7) << 7) + ((d & 31) << 2) + ((d >> 5) & 3); };
         float4 gam[Q8_XREG];
-        const bool in_regs = n4 <= Q8_XREG * RG_NW * 32;
+        const bool in_regs = d4 <= Q8_XREG * RG_NW * 32;
 #pragma unroll
         for (int it = 0; it < Q8_XREG; ++it) {
             const int d = threadIdx.x + it * RG_NW * 32;
-            gam[it] = (a.gamma != nullptr && in_regs && d < n4) ? __ldg(reinterpret_cast<const float4*>(a.gamma) + source_of(d))
+            gam[it] = (a.gamma != nullptr && in_regs && source_of(d) < n4) ? __ldg(reinterpret_cast<const float4*>(a.gamma) + source_of(d))
                                                                 : make_float4(1.f, 1.f, 1.f, 1.f);
         }
         pdl_wait();
@@ -434,17 +445,17 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
         float4* dst = reinterpret_cast<float4*>(xs);
         if (a.gamma == nullptr && !in_regs) {
             // a wide row without a norm (the FFN's down projection): eight loads in flight per thread
-            for (int base = threadIdx.x; base < n4; base += 8 * RG_NW * 32) {
+            for (int base = threadIdx.x; base < d4; base += 8 * RG_NW * 32) {
                 float4 t[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int d = base + u * RG_NW * 32;
-                    t[u] = d < n4 ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    t[u] = source_of(d) < n4 ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int d = base + u * RG_NW * 32;
-                    if (d < n4) dst[d] = t[u];
+                    if (d < d4) dst[d] = t[u];
                 }
             }
         }
@@ -452,7 +463,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
 #pragma unroll
         for (int it = 0; it < Q8_XREG; ++it) {
             const int d = threadIdx.x + it * RG_NW * 32;
-            xr[it] = (in_regs && d < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xr[it] = (in_regs && source_of(d) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         double inv_rms = 1.0;
         if (a.gamma != nullptr) {
@@ -488,12 +499,13 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
 #pragma unroll
             for (int it = 0; it < Q8_XREG; ++it) {
                 const int d = threadIdx.x + it * RG_NW * 32;
-                if (d < n4) dst[d] = a.gamma != nullptr ? normed(xr[it], gam[it]) : xr[it];
+                if (d < d4) dst[d] = a.gamma != nullptr ? normed(xr[it], gam[it]) : xr[it];
             }
         } else if (a.gamma != nullptr) {
-            for (int d = threadIdx.x; d < n4; d += RG_NW * 32) {
+            for (int d = threadIdx.x; d < d4; d += RG_NW * 32) {
                 const int sidx = source_of(d);
-                dst[d] = normed(__ldcg(src + sidx), __ldg(reinterpret_cast<const float4*>(a.gamma) + sidx));
+                dst[d] = sidx < n4 ? normed(__ldcg(src + sidx), __ldg(reinterpret_cast<const float4*>(a.gamma) + sidx))
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(RG_NW * 32) : "memory");
@@ -510,6 +522,8 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
             for (int c = 0; c < RG_COLS; ++c) acc[c] = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
+                if ((seg * 4 + j) * Q8_CHUNK >= Kp) break;
+                const bool in = seg * Q8_SEG + j * Q8_CHUNK + lane * 16 < a.K;   // past the end: x is zero, the scale made so
                 ulonglong2 xv[4];   // 16 activations of this lane as packed pairs
 #pragma unroll
                 for (int jj = 0; jj < 4; ++jj)
@@ -517,7 +531,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
 #pragma unroll
                 for (int c = 0; c < RG_COLS; ++c) {
                     const uint4 w = *reinterpret_cast<const uint4*>(st + c * Q8_SEG + j * Q8_CHUNK + lane * 16);
-                    const float scale = sc[c * (Q8_SEG / 32) + j * (Q8_CHUNK / 32) + (lane >> 1)];
+                    const float scale = in ? sc[c * (Q8_SEG / 32) + j * (Q8_CHUNK / 32) + (lane >> 1)] : 0.0f;
                     const unsigned words[4] = {w.x ^ 0x80808080u, w.y ^ 0x80808080u, w.z ^ 0x80808080u, w.w ^ 0x80808080u};
                     f32x2 p2 = 0ull;
 #pragma unroll
@@ -583,8 +597,8 @@ cudaError_t launch_ring(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     int ctas = quads < sm_count * RG_CTAS_PER_SM ? quads : sm_count * RG_CTAS_PER_SM;
     const int qpc = (quads + ctas - 1) / ctas;
     ctas = (quads + qpc - 1) / qpc;
-    const int nseg = a.K / Q8_SEG, vmul = SWIGLU ? 2 : 1;
-    const size_t smem = (size_t)NS * RG_STAGE + (size_t)a.K * 4 + (size_t)qpc * vmul * nseg * RG_COLS * 4 + 2 * NS * 8 + RG_NW * 8 + 16;
+    const int nseg = segments(a.K), vmul = SWIGLU ? 2 : 1;
+    const size_t smem = (size_t)NS * RG_STAGE + (size_t)padded_k(a.K) * 4 + (size_t)qpc * vmul * nseg * RG_COLS * 4 + 2 * NS * 8 + RG_NW * 8 + 16;
     auto kern = q8_gemv_ring_kernel<NS, SWIGLU>;
     static std::atomic<unsigned long long> configured{0};   // bit per device
     int dev = 0;
@@ -613,6 +627,7 @@ constexpr int RG_NS = 8;   // ring stages (a multiple of the consumer warps): 72
 
 bool ring_ok(const Q8GemvArgs& a, int sm_count) {
     if (a.M != 1 || !q8_fast_path(a.K) || a.N % RG_COLS != 0) return false;
+    if (((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(a.scales2)) & 15u) != 0) return false;   // bulk copies
     // Long streams (the lm_head, 295 MB at a 128 K vocabulary) run faster through the register
     // kernel (4.6 against 3.8 TB/s measured); the ring pays off where a kernel is short and its
     // first 72 KB per CTA are already on chip when the activations arrive.
@@ -620,12 +635,12 @@ bool ring_ok(const Q8GemvArgs& a, int sm_count) {
     const int quads = a.N / RG_COLS;
     const int ctas = quads < sm_count * RG_CTAS_PER_SM ? quads : sm_count * RG_CTAS_PER_SM;
     const int qpc = (quads + ctas - 1) / ctas;
-    const size_t smem = (size_t)RG_NS * RG_STAGE + (size_t)a.K * 4 + (size_t)qpc * (a.q2 ? 2 : 1) * (a.K / Q8_SEG) * RG_COLS * 4 + 512;
+    const size_t smem = (size_t)RG_NS * RG_STAGE + (size_t)padded_k(a.K) * 4 + (size_t)qpc * (a.q2 ? 2 : 1) * segments(a.K) * RG_COLS * 4 + 512;
     return smem <= 200 * 1024;
 }
 
 // Any K (ragged last block included), any N: one warp per output element.  Small shapes
-// of tests and models whose K is not a multiple of 2048; not a tuned path.
+// of tests and models whose K is not a multiple of 128; not a tuned path.
 template <bool SWIGLU>
 __global__ void __launch_bounds__(Q8_THREADS) q8_gemv_generic_kernel(Q8GemvArgs a) {
     extern __shared__ __align__(16) float q8_xs[];   // [K] activations of row blockIdx.y (normalised if asked)
@@ -742,9 +757,9 @@ cudaError_t launch_pdl(Kern kernel, dim3 grid, dim3 block, size_t smem, cudaStre
 
 template <int MB, bool SWIGLU>
 cudaError_t launch_fast(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
-    const size_t smem = (size_t)MB * a.K * sizeof(float);
+    const size_t smem = (size_t)MB * padded_k(a.K) * sizeof(float);
     auto kern = q8_gemv_kernel<MB, SWIGLU>;
-    if (smem > 48 * 1024) {
+    if (smem > 47 * 1024) {   // beside the static shared memory
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
@@ -758,7 +773,7 @@ cudaError_t launch_fast(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
 
 }  // namespace
 
-bool q8_fast_path(int K) { return K > 0 && K % Q8_SEG == 0 && (size_t)K * sizeof(float) <= 200 * 1024; }
+bool q8_fast_path(int K) { return K > 0 && K % 128 == 0 && (size_t)padded_k(K) * sizeof(float) <= 200 * 1024; }
 
 cudaError_t launch_q8_gemv(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;
@@ -768,8 +783,8 @@ cudaError_t launch_q8_gemv(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
         (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0 && (a.gamma == nullptr || (reinterpret_cast<uintptr_t>(a.gamma) & 15u) == 0)) {
         if (ring_ok(a, sm_count)) return swiglu ? launch_ring<RG_NS, true>(a, sm_count, s) : launch_ring<RG_NS, false>(a, sm_count, s);
         // Rows are taken four at a time while that fits shared memory; a row tile re-reads the weights.
-        const bool four = a.M >= 3 && (size_t)4 * a.K * sizeof(float) <= 160 * 1024;
-        const bool two = !four && a.M >= 2 && (size_t)2 * a.K * sizeof(float) <= 160 * 1024;
+        const bool four = a.M >= 3 && (size_t)4 * padded_k(a.K) * sizeof(float) <= 160 * 1024;
+        const bool two = !four && a.M >= 2 && (size_t)2 * padded_k(a.K) * sizeof(float) <= 160 * 1024;
         if (swiglu) {
             if (four) return launch_fast<4, true>(a, sm_count, s);
             if (two) return launch_fast<2, true>(a, sm_count, s);
@@ -784,13 +799,13 @@ cudaError_t launch_q8_gemv(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     int gx = (a.N + Q8_WARPS - 1) / Q8_WARPS;
     if (gx > sm_count * 4) gx = sm_count * 4;
     if (swiglu) {
-        if (smem > 48 * 1024) {
+        if (smem > 47 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(q8_gemv_generic_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
         }
         return launch_pdl(q8_gemv_generic_kernel<true>, dim3(gx, a.M), dim3(Q8_THREADS), smem, s, a);
     }
-    if (smem > 48 * 1024) {
+    if (smem > 47 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(q8_gemv_generic_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
