@@ -160,5 +160,5 @@ def test_pair_of_ctas_at_head_dim_64(ctx, G, T, pre):
         one = g1.forward_cached(q, k, v, flags or S.F_TENSOR)
     assert rel_err(got, ref) <= PREFILL_TOL, rel_err(got, ref)
     assert rel_err(one, ref) <= PREFILL_TOL, rel_err(one, ref)
-    assert not np.array_equal(got, one)
+    assert pre + T <= 64 or not np.array_equal(got, one)   # up to 64 positions both kernels sum alike
     g.close(); g1.close()
