@@ -98,10 +98,10 @@ __host__ __device__ constexpr int segments(int K) { return (K + Q8_SEG - 1) / Q8
 
 constexpr int Q8_XREG = 4;   // covers K <= 4096 from registers; wider rows re-read x from L2
 
-template <int MB>
+template <int MB, bool EVEN>
 __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows, float* xs, double* red,
                                            const float4 (&gam)[Q8_XREG]) {
-    const int n4 = a.K >> 2, K = padded_k(a.K), d4 = K >> 2;   // float4 of a row, and of its image in shared memory
+    const int n4 = a.K >> 2, K = EVEN ? a.K : padded_k(a.K), d4 = K >> 2;   // float4 of a row, and of its image in shared memory
     const bool in_regs = d4 <= Q8_XREG * Q8_THREADS;
     for (int m = 0; m < MB; ++m) {
         const bool live = m < rows;
@@ -181,7 +181,7 @@ struct Unit {
     float s[2][4];   // their block scales
 };
 
-template <bool SWIGLU>
+template <bool SWIGLU, bool EVEN>
 __device__ __forceinline__ void load_unit(const Q8GemvArgs& a, int pair, int seg, int lane, Unit& u) {
     const int kb = a.K >> 5;
 #pragma unroll
@@ -194,18 +194,18 @@ __device__ __forceinline__ void load_unit(const Q8GemvArgs& a, int pair, int seg
         const float* srow = sbase + (size_t)(valid ? n : 0) * kb + seg * (Q8_SEG / 32) + (lane >> 1);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const bool in = valid && seg * Q8_SEG + j * Q8_CHUNK + lane * 16 < a.K;   // past the end: zero scales (and x)
+            const bool in = valid && (EVEN || seg * Q8_SEG + j * Q8_CHUNK + lane * 16 < a.K);   // past the end: zero scales (and x)
             u.w[c][j] = in ? ldg_stream_v4(qrow + j * Q8_CHUNK) : make_uint4(0u, 0u, 0u, 0u);
             u.s[c][j] = in ? __ldg(srow + j * (Q8_CHUNK / 32)) : 0.0f;
         }
     }
 }
 
-template <int MB>
+template <int MB, bool EVEN>
 __device__ __forceinline__ void consume_unit(const Unit& u, const float* xs, int K, int seg, int lane, float (&acc)[MB][2]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if ((seg * 4 + j) * Q8_CHUNK >= K) break;   // K: the padded row length
+        if (!EVEN && (seg * 4 + j) * Q8_CHUNK >= K) break;   // K: the padded row length
         float4 xv[MB][4];
 #pragma unroll
         for (int m = 0; m < MB; ++m)
@@ -238,7 +238,8 @@ __device__ __forceinline__ void consume_unit(const Unit& u, const float* xs, int
 }
 
 // y[m0 .. m0+MB) x all N columns; gridDim.y walks the row tiles.
-template <int MB, bool SWIGLU>
+// EVEN: K is a multiple of the segment.
+template <int MB, bool SWIGLU, bool EVEN>
 __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8GemvArgs a) {
     extern __shared__ __align__(16) float q8_xs[];   // [MB][K] permuted activations
     __shared__ double red[Q8_WARPS];
@@ -246,13 +247,13 @@ __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * MB;
     const int rows = min(MB, a.M - m0);
-    const int nseg = segments(a.K);
+    const int nseg = EVEN ? a.K / Q8_SEG : segments(a.K);
     const int pairs = SWIGLU ? a.N : (a.N + 1) / 2;
     const int gw = blockIdx.x * Q8_WARPS + warp, tw = gridDim.x * Q8_WARPS;
 
     // weights first: they do not depend on the kernel ahead in the stream
     Unit cur;
-    if (gw < pairs) load_unit<SWIGLU>(a, gw, 0, lane, cur);
+    if (gw < pairs) load_unit<SWIGLU, EVEN>(a, gw, 0, lane, cur);
     float4 gam[Q8_XREG];   // norm weights of this thread's slots of a row: constants too
 #pragma unroll
     for (int it = 0; it < Q8_XREG; ++it) {
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8
     pdl_wait();
     pdl_launch_dependents();
     if (threadIdx.x < 4) best_sh[threadIdx.x] = 0ull;
-    stage_rows<MB>(a, m0, rows, q8_xs, red, gam);
+    stage_rows<MB, EVEN>(a, m0, rows, q8_xs, red, gam);
 
     unsigned long long best[MB];
 #pragma unroll
@@ -284,8 +285,8 @@ __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8
             const bool more_seg = seg + 1 < nseg;
             const int npair = more_seg ? pair : pair + tw;
             const bool have_next = npair < pairs;
-            if (have_next) load_unit<SWIGLU>(a, npair, more_seg ? seg + 1 : 0, lane, nxt);
-            consume_unit<MB>(cur, q8_xs, padded_k(a.K), seg, lane, acc);
+            if (have_next) load_unit<SWIGLU, EVEN>(a, npair, more_seg ? seg + 1 : 0, lane, nxt);
+            consume_unit<MB, EVEN>(cur, q8_xs, EVEN ? a.K : padded_k(a.K), seg, lane, acc);
             if (have_next) cur = nxt;
         }
 #pragma unroll
@@ -372,13 +373,13 @@ __device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) {
     return d;
 }
 
-template <int NS, bool SWIGLU>
+template <int NS, bool SWIGLU, bool EVEN>   // EVEN: K is a multiple of the segment
 __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs a, int quads_per_cta) {
     extern __shared__ __align__(128) unsigned char rg_raw[];
     unsigned char* ring = rg_raw;                                             // [NS][RG_STAGE]
-    const int Kp = padded_k(a.K);
+    const int Kp = EVEN ? a.K : padded_k(a.K);
     float* xs = reinterpret_cast<float*>(rg_raw + (size_t)NS * RG_STAGE);     // [Kp] permuted activations
-    const int nseg = segments(a.K);
+    const int nseg = EVEN ? a.K / Q8_SEG : segments(a.K);
     const int vmul = SWIGLU ? 2 : 1;
     float* part = xs + Kp;                                                   // [local stages][RG_COLS]
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(part + (size_t)quads_per_cta * vmul * nseg * RG_COLS);
@@ -409,7 +410,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
         const signed char* qb = (second ? a.q2 : a.q) + (size_t)quad * RG_COLS * a.K + (size_t)seg * Q8_SEG;
         const float* sb = (second ? a.scales2 : a.scales) + (size_t)quad * RG_COLS * (a.K >> 5) + seg * (Q8_SEG / 32);
         unsigned char* st = ring + (size_t)slot * RG_STAGE;
-        const uint32_t n = min(Q8_SEG, a.K - seg * Q8_SEG);   // the last segment of a row may be short
+        const uint32_t n = EVEN ? Q8_SEG : min(Q8_SEG, a.K - seg * Q8_SEG);   // the last segment of a row may be short
         mbar_arrive_expect_tx(&full_bar[slot], RG_COLS * (n + n / 8));
 #pragma unroll
         for (int c = 0; c < RG_COLS; ++c) {
@@ -522,8 +523,8 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
             for (int c = 0; c < RG_COLS; ++c) acc[c] = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if ((seg * 4 + j) * Q8_CHUNK >= Kp) break;
-                const bool in = seg * Q8_SEG + j * Q8_CHUNK + lane * 16 < a.K;   // past the end: x is zero, the scale made so
+                if (!EVEN && (seg * 4 + j) * Q8_CHUNK >= Kp) break;
+                const bool in = EVEN || seg * Q8_SEG + j * Q8_CHUNK + lane * 16 < a.K;   // past the end: x is zero, the scale made so
                 ulonglong2 xv[4];   // 16 activations of this lane as packed pairs
 #pragma unroll
                 for (int jj = 0; jj < 4; ++jj)
@@ -591,15 +592,15 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
     }
 }
 
-template <int NS, bool SWIGLU>
-cudaError_t launch_ring(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
+template <int NS, bool SWIGLU, bool EVEN>
+cudaError_t launch_ring_k(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     const int quads = a.N / RG_COLS;
     int ctas = quads < sm_count * RG_CTAS_PER_SM ? quads : sm_count * RG_CTAS_PER_SM;
     const int qpc = (quads + ctas - 1) / ctas;
     ctas = (quads + qpc - 1) / qpc;
     const int nseg = segments(a.K), vmul = SWIGLU ? 2 : 1;
     const size_t smem = (size_t)NS * RG_STAGE + (size_t)padded_k(a.K) * 4 + (size_t)qpc * vmul * nseg * RG_COLS * 4 + 2 * NS * 8 + RG_NW * 8 + 16;
-    auto kern = q8_gemv_ring_kernel<NS, SWIGLU>;
+    auto kern = q8_gemv_ring_kernel<NS, SWIGLU, EVEN>;
     static std::atomic<unsigned long long> configured{0};   // bit per device
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -621,6 +622,12 @@ cudaError_t launch_ring(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, a, qpc);
+}
+
+template <int NS, bool SWIGLU>
+cudaError_t launch_ring(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
+    // the checks for a short last segment cost 1.4 % of a 16-layer decode step where there is none
+    return a.K % Q8_SEG == 0 ? launch_ring_k<NS, SWIGLU, true>(a, sm_count, s) : launch_ring_k<NS, SWIGLU, false>(a, sm_count, s);
 }
 
 constexpr int RG_NS = 8;   // ring stages (a multiple of the consumer warps): 72 KB
@@ -758,7 +765,7 @@ cudaError_t launch_pdl(Kern kernel, dim3 grid, dim3 block, size_t smem, cudaStre
 template <int MB, bool SWIGLU>
 cudaError_t launch_fast(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     const size_t smem = (size_t)MB * padded_k(a.K) * sizeof(float);
-    auto kern = q8_gemv_kernel<MB, SWIGLU>;
+    auto kern = a.K % Q8_SEG == 0 ? q8_gemv_kernel<MB, SWIGLU, true> : q8_gemv_kernel<MB, SWIGLU, false>;
     if (smem > 47 * 1024) {   // beside the static shared memory
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
