@@ -141,14 +141,21 @@ int gemv(shainet_attn_ctx* ctx, const float* x, const signed char* q, const floa
     return SHAINET_ATTN_OK;
 }
 
-// Tensor-core product of planes [3][M][K] with one or two weights (their columns beside each other) into `out`.  Where
+// ctx->planes of M rows: their scales (padded, so that the planes behind them are aligned for TMA), then [2][M][K] halves.
+constexpr size_t scale_floats(size_t M) { return (M + 63) / 64 * 64; }
+constexpr size_t planes_floats(size_t M, size_t K) { return scale_floats(M) + M * K; }
+__half* planes_of(shainet_attn_ctx* ctx, int M) { return reinterpret_cast<__half*>(ctx->planes.p + scale_floats(M)); }
+constexpr int MAX_PLANE_K = 50 * 1024;   // a row is held in shared memory while its planes are made
+
+// Tensor-core product of planes [2][M][K] with one or two weights (their columns beside each other) into `out`.  Where
 // the plan splits the contraction: the splits are added into `out` (defer == null), or left in ctx->gemm_part
 // [splits][M][N] for the caller, who finds their number in *defer (1: `out` is complete).
 int gemm_tc(shainet_attn_ctx* ctx, const Q8Maps* w0, const Q8Maps* w1, int M, int K, const Q8GemmOut& out, int* defer, cudaStream_t s) {
     const int N = w0->N + (w1 ? w1->N : 0);
     const Q8GemmPlan plan = q8_gemm_plan(M, K, w0->N, w1 ? w1->N : 0, ctx->sm_count);
     Q8GemmArgs g{};
-    g.planes = reinterpret_cast<const __nv_bfloat16*>(ctx->planes.p);
+    g.planes = planes_of(ctx, M);
+    g.row_scale = ctx->planes.p;
     g.w[0] = w0;
     g.w[1] = w1;
     g.M = M;
@@ -175,13 +182,14 @@ int planes_acquire(shainet_attn_ctx* ctx, cudaStream_t s) {
     return SHAINET_ATTN_OK;
 }
 
-// Rows x [M, K] (RMS-normalised with gamma unless it is null) as the bfloat16 planes gemm_tc reads.
+// Rows x [M, K] (RMS-normalised with gamma unless it is null) as the planes gemm_tc reads.
 int make_planes(shainet_attn_ctx* ctx, const float* x, int M, int K, const float* gamma, double eps, cudaStream_t s) {
     Q8RowsArgs r{};
     r.x = x;
     r.gamma = gamma;
     r.eps = eps;
-    r.planes = reinterpret_cast<__nv_bfloat16*>(ctx->planes.p);
+    r.planes = planes_of(ctx, M);
+    r.row_scale = ctx->planes.p;
     r.M = M;
     r.K = K;
     CU(launch_q8_rows(r, s));
@@ -190,7 +198,6 @@ int make_planes(shainet_attn_ctx* ctx, const float* x, int M, int K, const float
 
 Q8GemmOut rows_out(float* y, int N, const float* residual) { return Q8GemmOut{{y}, {0}, {N}, 1, 0, residual}; }
 
-constexpr size_t planes_floats(size_t M, size_t K) { return (3 * M * K + 1) / 2; }
 
 enum { ACT_QKV = 0, ACT_ATTN = 1, ACT_H = 2, ACT_HIDDEN = 3, ACT_A = 4, ACT_B = 5 };
 
@@ -199,6 +206,7 @@ enum { ACT_QKV = 0, ACT_ATTN = 1, ACT_H = 2, ACT_HIDDEN = 3, ACT_A = 4, ACT_B = 
 bool few_rows(int M, int K) { return M <= 4 && q8_fast_path(K); }
 
 bool block_tensor_path(const shainet_attn_block* b, int T) {
+    if (std::max(std::max(b->d_model, b->q_dim), b->gate ? b->ffn : 0) > MAX_PLANE_K) return false;
     if (few_rows(T, b->d_model) && few_rows(T, b->q_dim) && (!b->gate || few_rows(T, b->ffn))) return false;
     return b->qkv_maps.ok && b->wo->maps.ok && (!b->gate || (b->gate->maps.ok && b->up->maps.ok && b->down->maps.ok));
 }
@@ -239,14 +247,15 @@ int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T,
     r.h = h;
     r.gamma = b->norm2;
     r.eps = b->eps;
-    r.planes = reinterpret_cast<__nv_bfloat16*>(ctx->planes.p);
+    r.planes = planes_of(ctx, T);
+    r.row_scale = ctx->planes.p;
     r.M = T;
     r.K = d;
     CU(launch_q8_rows(r, s));
     rc = gemm_tc(ctx, &b->gate->maps, &b->up->maps, T, d, rows_out(ctx->gate_up.p, 2 * b->ffn, nullptr), &splits, s);
     if (rc) return rc;
     CU(launch_q8_swiglu(splits > 1 ? ctx->gemm_part.p : ctx->gate_up.p, splits, (size_t)T * 2 * b->ffn, T, b->ffn,
-                        reinterpret_cast<__nv_bfloat16*>(ctx->planes.p), s));
+                        planes_of(ctx, T), ctx->planes.p, ctx->sm_count, s));
     return gemm_tc(ctx, &b->down->maps, nullptr, T, b->ffn, rows_out(out, d, h), nullptr, s);
 }
 
@@ -406,7 +415,7 @@ int shainet_attn_q8_gemv_dev(shainet_attn_ctx* ctx, const shainet_attn_q8* w, co
     if (M < 0) return fail(SHAINET_ATTN_E_INVALID, "negative row count");
     DeviceGuard g(ctx->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    if (M > 1 && !few_rows(M, w->K) && w->maps.ok && aligned16(x_dev)) {
+    if (M > 1 && !few_rows(M, w->K) && w->maps.ok && w->K <= MAX_PLANE_K && aligned16(x_dev)) {
         int rc = planes_acquire(ctx, s);
         if (!rc) rc = grow(ctx->planes, planes_floats(M, w->K), s);
         if (!rc) rc = make_planes(ctx, x_dev, M, w->K, nullptr, 0.0, s);

@@ -29,7 +29,7 @@ struct shainet_attn_ctx {
     cudaStream_t stream = nullptr;
     shainet::DevBuf q_rot, part, part_words, dev_in, dev_out;
     shainet::DevBuf kv_f32;             // fp32 image of a bfloat16 cache's rows, for the kernels that read fp32 caches only
-    shainet::DevBuf planes, gemm_part, gate_up;   // bfloat16 planes, split-K partials and raw gate|up products of the tensor-core projections
+    shainet::DevBuf planes, gemm_part, gate_up;   // row scales and planes, split-K partials and raw gate|up products of the tensor-core projections
     // q8_gemv_dev may be called on any stream: the newest such use of these buffers, which a use on another stream waits for
     cudaStream_t planes_stream = nullptr;
     cudaEvent_t planes_ev = nullptr;

@@ -1,8 +1,8 @@
 """Q8_0 products with several activation rows on the tensor cores, against an f64 product with the dequantised weight.
 
-Tolerance: the products are exact (int8 weights are bfloat16 values, an fp32 activation is the sum of three of them), what
-is left are fp32 sums of K <= 8192 terms; with the error normalised by the largest output, sqrt(K) 2^-24 times a few for
-the tensor core's truncating adds stays below 1e-5, the tolerance of the single-row kernels."""
+Tolerance: int8 weights are exact halves, an fp32 activation is the sum of two halves up to 2^-24 of it (or 2^-29 of its row's
+largest), what else is left are fp32 sums of K <= 8192 terms; with the error normalised by the largest output, sqrt(K) 2^-24
+times a few for the tensor core's truncating adds stays below 1e-5, the tolerance of the single-row kernels."""
 import numpy as np
 import pytest
 
@@ -47,4 +47,38 @@ def test_several_rows_against_f64(ctx, K, N, M):
     got = ty.cpu().numpy()
     assert np.isfinite(got[:M]).all() and np.isnan(got[M]).all()
     assert rel_err(got[:M], truth) <= DECODE_TOL, rel_err(got[:M], truth)
+    W.close()
+
+
+@pytest.mark.parametrize("M", [16, 64, 200])   # planes side by side, and passes of their own
+@pytest.mark.parametrize("K", [2048, 8192])
+def test_error_is_that_of_fp32_sums(ctx, K, M):
+    """2-norm of the error over that of the result: the row kernels' 1.04e-7 and 1.21e-7 (K = 2048, 8192) with a tenth of
+    room, on normal activations; and rows of very different magnitude, zeros, infinities and NaN keep to themselves."""
+    import torch
+    import shainet_b200 as S
+    rng = np.random.default_rng(K + M)
+    N = 512
+    q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+    s = (0.001 * rng.random((N, K // 32))).astype(np.float32)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    x[1] *= np.float32(2.0 ** 100)
+    x[2] *= np.float32(2.0 ** -100)
+    x[3] = 0.0
+    x[4, 7] = np.inf
+    x[5, 9] = np.nan
+    W = S.Q8Weight.from_quantized(ctx, q, s)
+    dev = torch.device("cuda:0")
+    tx = torch.from_numpy(x).to(dev)
+    ty = torch.empty((M, N), device=dev)
+    torch.cuda.synchronize()
+    W.gemv_dev(tx.data_ptr(), ty.data_ptr(), M)
+    ctx.sync()
+    truth = x.astype(np.float64) @ (q.astype(np.float64) * s.astype(np.float64).repeat(32, 1)).T
+    got = ty.cpu().numpy().astype(np.float64)
+    plain = [i for i in range(M) if i not in (3, 4, 5)]
+    for rows in (plain[:1], [1], [2], plain[3:]):
+        err = np.linalg.norm(got[rows] - truth[rows]) / np.linalg.norm(truth[rows])
+        assert err <= {2048: 1.15e-7, 8192: 1.33e-7}[K] * (1.0 if len(rows) > 1 else 1.2), (rows[0], err)
+    assert (got[3] == 0).all() and not np.isfinite(got[4]).any() and np.isnan(got[5]).all()
     W.close()
