@@ -205,18 +205,8 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_append_hd_kernel(PrepArgs a
         mbar_init(bar, 1);
         fence_mbar_init();
     }
-    __syncthreads();
-    chain_wait_and_release();
-    if (threadIdx.x == 0) {
-        mbar_arrive_expect_tx(bar, (uint32_t)per_row * HD * 4);
-        for (int slot = 0; slot < per_row; ++slot) {
-            const float* src = slot < H ? a.q + ((size_t)r * H + slot) * HD
-                             : slot < H + KV ? a.k_new + ((size_t)r * KV + (slot - H)) * HD
-                                             : a.v_new + ((size_t)r * KV + (slot - H - KV)) * HD;
-            bulk_g2s(buf + (size_t)slot * STRIDE, src, (uint32_t)HD * 4, bar);
-        }
-    }
-    // this lane's rotation pairs (i, i + HALF), i = lane + 32 k: angle, norm weights
+    // this lane's rotation pairs (i, i + HALF), i = lane + 32 k: angle, norm weights; constants,
+    // so before the wait for the kernel ahead
     float cs[PL], sn[PL], wq0[PL], wq1[PL], wk0[PL], wk1[PL];
 #pragma unroll
     for (int k = 0; k < PL; ++k) {
@@ -226,6 +216,18 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_append_hd_kernel(PrepArgs a
         wq1[k] = a.q_norm ? a.q_norm[i + HALF] : 1.0f;
         wk0[k] = a.k_norm ? a.k_norm[i] : 1.0f;
         wk1[k] = a.k_norm ? a.k_norm[i + HALF] : 1.0f;
+    }
+    __syncthreads();
+    chain_wait_and_release();
+    if (warp == 0) {   // one copy per head, issued by the lanes side by side
+        if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)per_row * HD * 4);
+        __syncwarp();
+        for (int slot = lane; slot < per_row; slot += 32) {
+            const float* src = slot < H ? a.q + ((size_t)r * H + slot) * HD
+                             : slot < H + KV ? a.k_new + ((size_t)r * KV + (slot - H)) * HD
+                                             : a.v_new + ((size_t)r * KV + (slot - H - KV)) * HD;
+            bulk_g2s(buf + (size_t)slot * STRIDE, src, (uint32_t)HD * 4, bar);
+        }
     }
     if (!mbar_wait(bar, 0, a.status, 31)) return;   // bounded; the whole CTA sees the same outcome
     if (a.b_q != nullptr || a.b_k != nullptr || a.b_v != nullptr) {
