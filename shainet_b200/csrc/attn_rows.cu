@@ -315,11 +315,10 @@ __global__ void __launch_bounds__(AR<HD, BM, ES>::THREADS, AR<HD, BM, ES>::CTAS)
 }
 
 // out = sum_s w_s o_s / sum_s w_s l_s over the splits, one warp per (row, query head): the weights are formed by the
-// lanes side by side, then HD/4 lanes walk the partials with eight loads in flight.
+// lanes side by side, HD/4 lanes walk the partials with eight to sixteen loads in flight.
 constexpr int CB_WARPS = 4;
 template <int HD>
 __global__ void __launch_bounds__(CB_WARPS * 32) attn_rows_combine_kernel(AttnArgs a) {
-    __shared__ float ws[CB_WARPS][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t hrow = (size_t)blockIdx.x * CB_WARPS + warp;
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -331,35 +330,40 @@ __global__ void __launch_bounds__(CB_WARPS * 32) attn_rows_combine_kernel(AttnAr
     if (ns <= 1) return;   // the split kernel wrote the row
     const float2* ml = reinterpret_cast<const float2*>(a.part_ml) + hrow * a.max_splits;
     const float* po = a.part_o + hrow * a.max_splits * HD;
-    float M = -INFINITY;
-    for (int s = lane; s < ns; s += 32) M = fmaxf(M, __ldcg(ml + s).x);
+    const bool on = lane < HD / 4;
+    auto partial = [&](int sp) {
+        return (on && sp < ns) ? __ldcg(reinterpret_cast<const float4*>(po + (size_t)sp * HD) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    // the first partials are requested together with the maxima that weigh them
+    float4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = partial(k);
+    const float2 first = lane < ns ? __ldcg(ml + lane) : make_float2(-INFINITY, 0.0f);
+    float M = first.x;
+    for (int s = 32 + lane; s < ns; s += 32) M = fmaxf(M, __ldcg(ml + s).x);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(FULL, M, off));
     float L = 0.0f;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool on = lane < HD / 4;
     for (int s0 = 0; s0 < ns; s0 += 32) {
         float w = 0.0f;
         if (s0 + lane < ns) {
-            const float2 v = __ldcg(ml + s0 + lane);
-            w = v.x == -INFINITY ? 0.0f : exp2f((v.x - M) * LOG2E);
-            L = fmaf(w, v.y, L);
+            const float2 p = s0 == 0 ? first : __ldcg(ml + s0 + lane);
+            w = p.x == -INFINITY ? 0.0f : exp2f((p.x - M) * LOG2E);
+            L = fmaf(w, p.y, L);
         }
-        __syncwarp();
-        ws[warp][lane] = w;
-        __syncwarp();
         const int n = min(32, ns - s0);
         for (int s1 = 0; s1 < n; s1 += 8) {
-            float4 v[8];
+            float4 nxt[8];   // the next eight, while these are added
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                v[k] = (on && s1 + k < n) ? __ldcg(reinterpret_cast<const float4*>(po + (size_t)(s0 + s1 + k) * HD) + lane)
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < 8; ++k) nxt[k] = partial(s0 + s1 + 8 + k);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const float wk = s1 + k < n ? ws[warp][s1 + k] : 0.0f;
+                const float wk = __shfl_sync(FULL, w, s1 + k);   // zero past the last split
                 acc = make_float4(fmaf(wk, v[k].x, acc.x), fmaf(wk, v[k].y, acc.y), fmaf(wk, v[k].z, acc.z), fmaf(wk, v[k].w, acc.w));
             }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = nxt[k];
         }
     }
 #pragma unroll
