@@ -253,6 +253,33 @@ void plan_splits(int sm_count, const HeadShape& hs, int rows, long long total_vi
     (void)rows;
 }
 
+// Batched decode: the smallest slice for which the slices of all sequences together are resident at once (0: none is worth
+// it).  Four waves of slices, the general plan, balance ragged sequences better, but each wave pays a CTA's prologue and
+// merge, 5 us and more.  One wave costs the rows by which its slice exceeds the even share, at about 45 ns a row at head_dim
+// 128 (6.5 TB/s over two CTAs an SM); it is taken where that is less than 16 us.  Per layer, one against four waves: 8 sequences of
+// 200 to 4000, head_dim 64: 25 / 33 us; 16 of 500 to 3000: 44 / 52; 3 of 16 to 32 thousand: 99 / 107; 32 of 2 to 16 thousand,
+// eight heads per kv head, bfloat16 (the slice 1.4 times the even share): 183 / 163, not taken.
+int plan_one_wave(int sm_count, const HeadShape& hs, const SeqDesc* seqs, int batch, long long total_visible, int max_visible, int kv_elem_bytes) {
+    const int tw = splitk_tile_rows(hs, kv_elem_bytes, true);
+    const long long slots = (long long)sm_count * splitk_ctas_per_sm(hs);
+    auto fits = [&](int tiles) {
+        const long long chunk = (long long)tiles * tw;
+        long long n = 0;
+        for (int b = 0; b < batch; ++b) n += (seqs[b].start + chunk) / chunk;   // slices of start + 1 rows
+        return n * hs.num_kv_heads <= slots;
+    };
+    const long long even = total_visible * hs.num_kv_heads / slots;
+    const long long limit = std::min<long long>(even + even * 8 / 100 + 350 * 128 / hs.head_dim, max_visible + tw);
+    int lo = 4, hi = std::max(4, (int)(limit / tw));   // from one tile per consumer warp
+    if (!fits(hi)) return 0;
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (fits(mid)) hi = mid;
+        else lo = mid + 1;
+    }
+    return hi * tw;
+}
+
 int run_attention_untimed(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seqs, int kv_elem_bytes, int batch, int T,
                           long long total_visible, int max_visible, const float* q_rot, float* out, float scale,
                           unsigned flags, cudaStream_t s);
@@ -351,7 +378,7 @@ bool single_token_rows(const shainet_attn_ctx* ctx, const HeadShape& hs, unsigne
 // `par` supplies the shared head shape, RoPE table, norm weights and biases.
 int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int batch, int T, long long total_visible,
              int max_visible, const float* q, const float* k_new, const float* v_new, float* out, float scale,
-             unsigned flags, cudaStream_t s, int pos_delta = 0, int no_append = 0) {
+             unsigned flags, cudaStream_t s, int pos_delta = 0, int no_append = 0, const SeqDesc* seqs_host = nullptr) {
     const HeadShape hs = par->hs;
     const bool fused = T == 1 && splitk_supported(hs) && !single_token_rows(ctx, hs, flags, pos_delta, no_append) &&
                        !(flags & (SHAINET_ATTN_F_GENERIC | SHAINET_ATTN_F_UNFUSED | SHAINET_ATTN_F_TENSOR));
@@ -430,6 +457,10 @@ int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int
     f.status = ctx->status_dev;
     plan_splits(ctx->sm_count, hs, batch, total_visible, max_visible, batch > 1 ? 4 : 1, &f.chunk_rows, &f.max_splits, par->es,
                 seqs.many != nullptr);
+    if (const int chunk = seqs_host ? plan_one_wave(ctx->sm_count, hs, seqs_host, batch, total_visible, max_visible, par->es) : 0) {
+        f.chunk_rows = chunk;
+        f.max_splits = (max_visible + chunk - 1) / chunk;
+    }
     f.max_groups = fused_merge_groups(f.max_splits);
     // A single sequence whose grid is fully resident merges through {value, epoch} words
     // (8 bytes per partial float) polled by the merging CTAs; batched decode keeps float
@@ -1263,7 +1294,7 @@ int shainet_attn_forward_batched_dev(shainet_attn_ctx* ctx, shainet_attn_kv* con
     CU(cudaEventRecord(ctx->seq_ev[slot], s));
     SeqRef seqs{};
     seqs.many = dd;
-    rc = run_step(ctx, first, seqs, batch, 1, total_visible, max_visible, q, k_new, v_new, out, scale, flags, s);
+    rc = run_step(ctx, first, seqs, batch, 1, total_visible, max_visible, q, k_new, v_new, out, scale, flags, s, 0, 0, hd);
     if (rc) return rc;
     for (int b = 0; b < batch; ++b) kvs[b]->len += 1;
     return SHAINET_ATTN_OK;
