@@ -432,8 +432,8 @@ int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int
             if (ctx->kv_f32.p != before) CU(cudaMemsetAsync(ctx->kv_f32.p, 0, ctx->kv_f32.cap * sizeof(float), s));
             float* wk = ctx->kv_f32.p;
             float* wv = wk + per;
-            CU(launch_kv_convert(seqs.one.k, par->es, seqs.one.capacity, wk, 4, cap_s, hs.num_kv_heads, hs.head_dim, 0, max_visible, s));
-            CU(launch_kv_convert(seqs.one.v, par->es, seqs.one.capacity, wv, 4, cap_s, hs.num_kv_heads, hs.head_dim, 0, max_visible, s));
+            CU(launch_kv_widen(seqs.one.k, seqs.one.v, seqs.one.capacity, wk, wv, cap_s, hs.num_kv_heads, hs.head_dim, seqs.one.start,
+                               max_visible, s));
             seqs.one = SeqDesc{wk, wv, seqs.one.start, cap_s};
         }
         return run_attention(ctx, hs, seqs, par->es, batch, T, total_visible, max_visible, ctx->q_rot.p, out, scale, flags, s);

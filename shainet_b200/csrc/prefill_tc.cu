@@ -463,6 +463,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     cluster_sync_all();   // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // q, the new rows and a widened cache come from the kernels ahead
 
     if (warp == 0) {
         // ---------------- TMA producer: this CTA's halves, reported to the leader's barriers ----------------
@@ -744,13 +745,15 @@ cudaError_t launch_pf_pair128(const AttnArgs& a, cudaStream_t s) {
     cfg.blockDim = dim3(C::THREADS);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // barriers and tensor memory are set up meanwhile
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, attn_prefill_pair_kernel<HD>, tq, tk, tv, p);
 }
 

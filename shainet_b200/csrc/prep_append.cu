@@ -402,7 +402,56 @@ __global__ void kv_convert_kernel(const void* src, int src_es, long long src_pit
     }
 }
 
+// Rows [0, rows) of a bfloat16 cache widened into the fp32 image, K and V in one launch: eight elements per load, four loads in
+// flight per thread.  The kernel ahead in the stream appends the rows from `start` on; the older ones, nearly all of
+// them, are widened while it still runs.
+constexpr int WIDEN_VECS = 4;
+__global__ void __launch_bounds__(256) kv_widen_kernel(const uint4* k, const uint4* v, float4* wk, float4* wv, long long src_pitch,
+                                                       long long dst_pitch, long long old_vecs, long long vecs) {
+    const uint4* src = (blockIdx.z ? v : k) + blockIdx.y * src_pitch;
+    float4* dst = (blockIdx.z ? wv : wk) + 2 * blockIdx.y * dst_pitch;
+    const long long i0 = (long long)blockIdx.x * (256 * WIDEN_VECS);
+    if (i0 + 256 * WIDEN_VECS > old_vecs) asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint4 w[WIDEN_VECS];
+#pragma unroll
+    for (int u = 0; u < WIDEN_VECS; ++u) {
+        const long long i = i0 + u * 256 + threadIdx.x;
+        w[u] = i < vecs ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < WIDEN_VECS; ++u) {
+        const long long i = i0 + u * 256 + threadIdx.x;
+        if (i < vecs) {   // a bfloat16 is the upper half of the fp32 of the same value
+            dst[2 * i] = make_float4(__uint_as_float(w[u].x << 16), __uint_as_float(w[u].x & 0xffff0000u), __uint_as_float(w[u].y << 16),
+                                     __uint_as_float(w[u].y & 0xffff0000u));
+            dst[2 * i + 1] = make_float4(__uint_as_float(w[u].z << 16), __uint_as_float(w[u].z & 0xffff0000u),
+                                         __uint_as_float(w[u].w << 16), __uint_as_float(w[u].w & 0xffff0000u));
+        }
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_kv_widen(const void* k, const void* v, int src_capacity, float* wk, float* wv, int dst_capacity, int num_kv_heads,
+                            int head_dim, int start, int rows, cudaStream_t s) {
+    if (rows <= 0 || num_kv_heads <= 0) return cudaSuccess;
+    if (head_dim % 8 != 0) {   // rows that are no whole number of 16-byte vectors
+        cudaError_t e = launch_kv_convert(k, 2, src_capacity, wk, 4, dst_capacity, num_kv_heads, head_dim, 0, rows, s);
+        return e != cudaSuccess ? e : launch_kv_convert(v, 2, src_capacity, wv, 4, dst_capacity, num_kv_heads, head_dim, 0, rows, s);
+    }
+    const long long per_row = head_dim / 8, vecs = per_row * rows;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((vecs + 256 * WIDEN_VECS - 1) / (256 * WIDEN_VECS)), num_kv_heads, 2);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kv_widen_kernel, static_cast<const uint4*>(k), static_cast<const uint4*>(v), reinterpret_cast<float4*>(wk),
+                              reinterpret_cast<float4*>(wv), per_row * src_capacity, per_row * dst_capacity, per_row * start, vecs);
+}
 
 cudaError_t launch_kv_convert(const void* src, int src_elem_bytes, int src_capacity, void* dst, int dst_elem_bytes,
                               int dst_capacity, int num_kv_heads, int head_dim, int row0, int rows, cudaStream_t s) {
