@@ -254,11 +254,11 @@ void plan_splits(int sm_count, const HeadShape& hs, int rows, long long total_vi
 }
 
 // Batched decode: the smallest slice for which the slices of all sequences together are resident at once (0: none is worth
-// it).  Four waves of slices, the general plan, balance ragged sequences better, but each wave pays a CTA's prologue and
-// merge, 5 us and more.  One wave costs the rows by which its slice exceeds the even share, at about 45 ns a row at head_dim
-// 128 (6.5 TB/s over two CTAs an SM); it is taken where that is less than 16 us.  Per layer, one against four waves: 8 sequences of
-// 200 to 4000, head_dim 64: 25 / 33 us; 16 of 500 to 3000: 44 / 52; 3 of 16 to 32 thousand: 99 / 107; 32 of 2 to 16 thousand,
-// eight heads per kv head, bfloat16 (the slice 1.4 times the even share): 183 / 163, not taken.
+// it).  Four waves of slices, the general plan, balance ragged sequences better, but their prologues and merges cost about
+// 10 us a launch more.  One wave costs the rows by which its slice exceeds the even share, at about 45 ns a row at
+// head_dim 128 (6.5 TB/s over two CTAs an SM): it is taken up to 200 of them.  Per layer, one against four waves: 8 sequences of
+// 200 to 4000, head_dim 64: 25 / 33 us; 16 of 500 to 3000: 44 / 52; 3 of 16 to 32 thousand: 99 / 107; past the line 6 of
+// 3 to 24 thousand: 103 / 91; 32 of 2 to 16 thousand, eight heads per kv head, bfloat16: 186 / 164.
 int plan_one_wave(int sm_count, const HeadShape& hs, const SeqDesc* seqs, int batch, long long total_visible, int max_visible, int kv_elem_bytes) {
     const int tw = splitk_tile_rows(hs, kv_elem_bytes, true);
     const long long slots = (long long)sm_count * splitk_ctas_per_sm(hs);
@@ -269,7 +269,7 @@ int plan_one_wave(int sm_count, const HeadShape& hs, const SeqDesc* seqs, int ba
         return n * hs.num_kv_heads <= slots;
     };
     const long long even = total_visible * hs.num_kv_heads / slots;
-    const long long limit = std::min<long long>(even + even * 8 / 100 + 350 * 128 / hs.head_dim, max_visible + tw);
+    const long long limit = std::min<long long>(even + 200 * 128 / hs.head_dim, max_visible + tw);
     int lo = 4, hi = std::max(4, (int)(limit / tw));   // from one tile per consumer warp
     if (!fits(hi)) return 0;
     while (lo < hi) {
