@@ -114,7 +114,7 @@ __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows
 #pragma unroll
         for (int it = 0; it < Q8_XREG; ++it) {
             const int d = threadIdx.x + it * Q8_THREADS;
-            xr[it] = (live && source_of(d) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xr[it] = (live && (EVEN ? d : source_of(d)) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (a.gamma == nullptr) {
             if (in_regs) {
@@ -125,7 +125,7 @@ __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows
                 }
             } else {
                 for (int d = threadIdx.x; d < d4; d += Q8_THREADS)
-                    dst[d] = (live && source_of(d) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    dst[d] = (live && (EVEN ? d : source_of(d)) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             continue;
         }
@@ -168,8 +168,8 @@ __device__ __forceinline__ void stage_rows(const Q8GemvArgs& a, int m0, int rows
         } else {
             for (int d = threadIdx.x; d < d4; d += Q8_THREADS) {
                 const int s = source_of(d);
-                const float4 v = (live && s < n4) ? __ldcg(src + s) : make_float4(0.f, 0.f, 0.f, 0.f);
-                dst[d] = s < n4 ? normed(v, __ldg(reinterpret_cast<const float4*>(a.gamma) + s)) : v;
+                const float4 v = (live && (EVEN || s < n4)) ? __ldcg(src + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+                dst[d] = (EVEN || s < n4) ? normed(v, __ldg(reinterpret_cast<const float4*>(a.gamma) + s)) : v;
             }
         }
     }
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(Q8_THREADS, MB == 1 ? 2 : 1) q8_gemv_kernel(Q8
     for (int it = 0; it < Q8_XREG; ++it) {
         const int d = threadIdx.x + it * Q8_THREADS;
         const int src = ((d >> 7) << 7) + ((d & 31) << 2) + ((d >> 5) & 3);
-        gam[it] = (a.gamma != nullptr && src < (a.K >> 2) && padded_k(a.K) <= 4 * Q8_XREG * Q8_THREADS)
+        gam[it] = (a.gamma != nullptr && (EVEN ? d : src) < (a.K >> 2) && (EVEN ? a.K : padded_k(a.K)) <= 4 * Q8_XREG * Q8_THREADS)
                       ? __ldg(reinterpret_cast<const float4*>(a.gamma) + src)
                       : make_float4(1.f, 1.f, 1.f, 1.f);
     }
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
 #pragma unroll
         for (int it = 0; it < Q8_XREG; ++it) {
             const int d = threadIdx.x + it * RG_NW * 32;
-            gam[it] = (a.gamma != nullptr && in_regs && source_of(d) < n4) ? __ldg(reinterpret_cast<const float4*>(a.gamma) + source_of(d))
+            gam[it] = (a.gamma != nullptr && in_regs && (EVEN ? d : source_of(d)) < n4) ? __ldg(reinterpret_cast<const float4*>(a.gamma) + source_of(d))
                                                                 : make_float4(1.f, 1.f, 1.f, 1.f);
         }
         pdl_wait();
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int d = base + u * RG_NW * 32;
-                    t[u] = source_of(d) < n4 ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    t[u] = (EVEN ? d : source_of(d)) < n4 ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
 #pragma unroll
         for (int it = 0; it < Q8_XREG; ++it) {
             const int d = threadIdx.x + it * RG_NW * 32;
-            xr[it] = (in_regs && source_of(d) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xr[it] = (in_regs && (EVEN ? d : source_of(d)) < n4) ? __ldcg(src + source_of(d)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         double inv_rms = 1.0;
         if (a.gamma != nullptr) {
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) q8_gemv_ring_kernel(Q8GemvArgs 
         } else if (a.gamma != nullptr) {
             for (int d = threadIdx.x; d < d4; d += RG_NW * 32) {
                 const int sidx = source_of(d);
-                dst[d] = sidx < n4 ? normed(__ldcg(src + sidx), __ldg(reinterpret_cast<const float4*>(a.gamma) + sidx))
+                dst[d] = (EVEN || sidx < n4) ? normed(__ldcg(src + sidx), __ldg(reinterpret_cast<const float4*>(a.gamma) + sidx))
                                    : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
