@@ -389,7 +389,13 @@ struct PFP {
     // tiles ahead of V.
     static constexpr int SB = 3;
     static constexpr int KS = 3, VS = 2;
-    static constexpr int XCHG_BYTES = 2 * 2 * BM * 4;   // [parity][half][row] row maxima; reused for the row sums
+    // At head_dim 64 a step is summed as the one-CTA kernel sums its two 64-position blocks, bit for bit: the running maximum
+    // follows block after block (the probabilities, and with them their TF32 truncation, depend on it: with one
+    // maximum per 128 positions results moved by 2e-4 of themselves), and so does the row sum.  500 tokens over 3500 bfloat16
+    // rows of the LLaMA-3.2-1B shape: 53 us a layer, 52 with one maximum.
+    static constexpr bool BLOCKS64 = HD == 64;
+    // [parity][half][row] row maxima, and with BLOCKS64 the sum of the half's probabilities in the step before; reused for the row sums
+    static constexpr int XCHG_BYTES = 2 * 2 * BM * (BLOCKS64 ? 8 : 4);
     static constexpr int BAR_BYTES = 256;
     static constexpr size_t SMEM_BYTES = Q_BYTES + KS * K_BYTES + VS * V_BYTES + XCHG_BYTES + BAR_BYTES;   // 1024-aligned base
     static constexpr int TMEM_S = 0;             // [buffer] score/probability blocks of BN columns
@@ -563,6 +569,11 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const uint32_t oa = tmem + lane_addr + C::TMEM_O + half * (HD / 2);   // this thread's half of the output columns
         const uint32_t p_leader = map_to_cta(smem_u32(&p_full[0]), 0u);   // the leader's p_full[0]; the others follow at 8 bytes
         float m = -INFINITY, l = 0.0f;
+        // BLOCKS64: this half's sum of the step before (exchanged one step late, with the maxima), the factor between the sums
+        // of its two blocks, and whether there is one
+        float part = 0.0f, l_alpha = 1.0f;
+        bool second = false;
+        auto add_step = [&](float other) { l = (l + (half ? other : part)) * l_alpha + (half ? part : other); };
         bool ok = true;
         for (int j = 0; j < n; ++j) {
             const int b = j % SB;
@@ -585,43 +596,95 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 #pragma unroll
             for (int c = 0; c < 32; ++c) mx = fmaxf(mx, fmaxf(__uint_as_float(s0[c]), __uint_as_float(s1[c])));
             // the row's maximum over both halves
-            float* xm = xchg + (size_t)(j & 1) * 2 * C::BM;
-            xm[half * C::BM + r] = mx;
-            mbar_arrive(&x_bar[quad]);
-            if (!(ok = mbar_wait(&x_bar[quad], j & 1, a.status, 59))) break;
-            mx = fmaxf(mx, xm[(half ^ 1) * C::BM + r]);
-            const float m_cand = fmaxf(m, mx * sl2);    // the positive factor commutes with max; identical in both halves
             bool o_seen = j == 0;
-            if (__any_sync(0xffffffffu, m_cand - m > C::RESCALE_STEP)) {   // always on the first step (m = -inf)
-                const float alpha = ex2_approx(m - m_cand);
-                m = m_cand;
-                l *= alpha;
-                if (j > 0) {
-                    if (!(ok = mbar_wait(o_done, (j - 1) & 1, a.status, 60))) break;
-                    o_seen = true;
-                    tc_fence_after();
-#pragma unroll
-                    for (int ch = 0; ch < HD / 64; ++ch) {
-                        uint32_t v[32];
-                        tmem_ld32(oa + ch * 32, v);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * alpha);
-                        tmem_st32(oa + ch * 32, v);
+            bool rescale;                       // of the accumulator, by alpha0 and then alpha1
+            float alpha0 = 1.0f, alpha1 = 1.0f;
+            float my_m;                         // the maximum this thread's probabilities are taken against
+            if constexpr (C::BLOCKS64) {
+                float2* xm = reinterpret_cast<float2*>(xchg) + (size_t)(j & 1) * 2 * C::BM;
+                xm[half * C::BM + r] = make_float2(mx, part);
+                mbar_arrive(&x_bar[quad]);
+                if (!(ok = mbar_wait(&x_bar[quad], j & 1, a.status, 59))) break;
+                const float2 other = xm[(half ^ 1) * C::BM + r];
+                add_step(other.y);
+                // identical in both halves; where the larger of the two blocks' maxima asks for no rescaling, neither block does
+                second = false;
+                rescale = __any_sync(0xffffffffu, fmaxf(mx, other.x) * sl2 - m > C::RESCALE_STEP);   // always on the first step (m = -inf)
+                my_m = m;
+                if (rescale) {
+                    const float m_first = fmaxf(m, (half ? other.x : mx) * sl2);
+                    if (__any_sync(0xffffffffu, m_first - m > C::RESCALE_STEP)) {
+                        alpha0 = ex2_approx(m - m_first);
+                        m = m_first;
+                        l *= alpha0;
+                        my_m = m;
                     }
+                    const float m_second = fmaxf(m, (half ? mx : other.x) * sl2);
+                    second = __any_sync(0xffffffffu, m_second - m > C::RESCALE_STEP);
+                    if (second) {
+                        alpha1 = ex2_approx(m - m_second);
+                        m = m_second;
+                        if (half) my_m = m;
+                    }
+                }
+                l_alpha = alpha1;
+            } else {
+                float* xm = xchg + (size_t)(j & 1) * 2 * C::BM;
+                xm[half * C::BM + r] = mx;
+                mbar_arrive(&x_bar[quad]);
+                if (!(ok = mbar_wait(&x_bar[quad], j & 1, a.status, 59))) break;
+                mx = fmaxf(mx, xm[(half ^ 1) * C::BM + r]);
+                const float m_cand = fmaxf(m, mx * sl2);    // the positive factor commutes with max; identical in both halves
+                rescale = __any_sync(0xffffffffu, m_cand - m > C::RESCALE_STEP);   // always on the first step (m = -inf)
+                if (rescale) {
+                    alpha0 = ex2_approx(m - m_cand);
+                    m = m_cand;
+                    l *= alpha0;
+                }
+                my_m = m;
+            }
+            if (rescale && j > 0) {
+                if (!(ok = mbar_wait(o_done, (j - 1) & 1, a.status, 60))) break;
+                o_seen = true;
+                tc_fence_after();
+#pragma unroll
+                for (int ch = 0; ch < HD / 64; ++ch) {
+                    uint32_t v[32];
+                    tmem_ld32(oa + ch * 32, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) {
+                        float x = __uint_as_float(v[c]) * alpha0;
+                        if constexpr (C::BLOCKS64) x *= alpha1;
+                        v[c] = __float_as_uint(x);
+                    }
+                    tmem_st32(oa + ch * 32, v);
                 }
             }
             float sum0 = 0.0f, sum1 = 0.0f;
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
-                const float p0 = ex2_approx(fmaf(__uint_as_float(s0[c]), sl2, -m));
-                const float p1 = ex2_approx(fmaf(__uint_as_float(s1[c]), sl2, -m));
+                const float p0 = ex2_approx(fmaf(__uint_as_float(s0[c]), sl2, -my_m));
+                const float p1 = ex2_approx(fmaf(__uint_as_float(s1[c]), sl2, -my_m));
                 s0[c] = __float_as_uint(p0);
                 s1[c] = __float_as_uint(p1);
                 sum0 += p0;
                 sum1 += p1;
             }
-            l += sum0 + sum1;
+            if constexpr (C::BLOCKS64) {
+                part = sum0 + sum1;
+                // Both blocks meet in one product.  The first one's probabilities take the second one's rescaling here, where the
+                // one-CTA kernel has it in the accumulator (the one place where the two are not bit for bit alike).
+                if (second && half == 0) {
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) {
+                        s0[c] = __float_as_uint(__uint_as_float(s0[c]) * alpha1);
+                        s1[c] = __float_as_uint(__uint_as_float(s1[c]) * alpha1);
+                    }
+                }
+            } else {
+                l += sum0 + sum1;
+            }
             tmem_st32(sa, s0);
             tmem_st32(sa + 32, s1);
             tmem_wait_st();
@@ -635,11 +698,17 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         if (ok && n > 0 && (ok = mbar_wait(o_done, (n - 1) & 1, a.status, 62))) {
             tc_fence_after();
             // the row's sum over both halves (same exchange, one more phase of the quadrant's barrier)
-            float* xl = xchg + (size_t)(n & 1) * 2 * C::BM;
-            xl[half * C::BM + r] = l;
+            float* xl = xchg + (size_t)(n & 1) * 2 * C::BM * (C::BLOCKS64 ? 2 : 1);
+            xl[half * C::BM + r] = C::BLOCKS64 ? part : l;
             mbar_arrive(&x_bar[quad]);
             if (mbar_wait(&x_bar[quad], n & 1, a.status, 63)) {
-                const float lt = l + xl[(half ^ 1) * C::BM + r];
+                float lt = l;
+                if constexpr (C::BLOCKS64) {
+                    add_step(xl[(half ^ 1) * C::BM + r]);
+                    lt = l;
+                } else {
+                    lt += xl[(half ^ 1) * C::BM + r];
+                }
                 const float inv = PF_TRUNC_GAIN * PF_TRUNC_GAIN / lt;   // V and P are both truncated by the tensor core
                 float* dst = a.out + ((size_t)(ti0 + r) * a.num_heads + head) * HD + half * (HD / 2);
 #pragma unroll
