@@ -41,7 +41,7 @@ extern "C" {
 /* forward flags */
 #define SHAINET_ATTN_F_GENERIC 1u  /* force the shape-agnostic kernel */
 #define SHAINET_ATTN_F_SPLITK 2u   /* force the split-K decode kernel (error if unsupported) */
-#define SHAINET_ATTN_F_TENSOR 4u   /* force the tcgen05 prefill kernel (error if unsupported); at head_dim 64 its one-CTA form */
+#define SHAINET_ATTN_F_TENSOR 4u   /* force the tcgen05 prefill kernel (error if unsupported) */
 #define SHAINET_ATTN_F_UNFUSED 8u  /* decode as three launches (RoPE/append, split-K, merge) instead of one */
 /* The caller vouches that q/k_new/v_new (device-pointer entries only) were
  * complete before the kernel launched immediately before this call on the same

@@ -318,9 +318,7 @@ int run_attention_untimed(shainet_attn_ctx* ctx, const HeadShape& hs, SeqRef seq
     a.hs = hs;
     a.scale = scale;
     a.status = ctx->status_dev;
-    // a call that forces the tensor kernel keeps, at head_dim 64, the one-CTA kernel and with it its results bit for bit;
-    // the pair is what the library chooses by itself
-    a.prefill_one_cta = (flags & SHAINET_ATTN_F_TENSOR_1CTA) || ((flags & SHAINET_ATTN_F_TENSOR) && hs.head_dim == 64) ? 1 : 0;
+    a.prefill_one_cta = (flags & SHAINET_ATTN_F_TENSOR_1CTA) ? 1 : 0;
     if (kern == Kernel::Generic) {
         if (hs.head_dim > 256) return fail(SHAINET_ATTN_E_UNSUPPORTED, "head_dim %d > 256", hs.head_dim);
         CU(launch_attn_generic(a, s));

@@ -100,7 +100,7 @@ def test_prefill_pairs_row_tiles_when_the_group_size_is_odd(ctx, H, KV, hd, T):
 
 @pytest.mark.parametrize("shape,T", [(Q8B, 700), (L1B, 384), (Q30, 257)], ids=["qwen3_8b_700", "llama1b_384", "qwen3_30b_257"])
 def test_cluster_pair_kernel_and_single_cta_kernel_against_the_oracle(ctx, shape, T):
-    """Even group sizes at head_dim 128 run on a cluster of two CTAs (two query heads of one kv head, one tensor-core tile
+    """Even group sizes run on a cluster of two CTAs (two query heads of one kv head, one tensor-core tile
     of 256 rows, 128-position steps); SHAINET_ATTN_F_TENSOR_1CTA keeps the one-CTA kernel (two tiles per CTA, 64-position steps).
     Both against the oracle, a first chunk and a second one over it; the two kernels also agree with each other
     far inside the tolerance (same TF32 products, different summation order)."""
@@ -116,7 +116,7 @@ def test_cluster_pair_kernel_and_single_cta_kernel_against_the_oracle(ctx, shape
         assert rel_err(pair, ref) <= PREFILL_TOL, (n, rel_err(pair, ref))
         assert rel_err(single, ref) <= PREFILL_TOL, (n, rel_err(single, ref))
         assert rel_err(pair, single) <= PREFILL_TOL / 2
-        # head_dim 128: two different kernels did run; head_dim 64 runs the one-CTA kernel either way
+        # head_dim 128: two different kernels did run; at head_dim 64 the pair sums its two blocks of 64 as the one-CTA kernel does
         assert np.array_equal(pair, single) == (shape["hd"] == 64)
     g.close(); g1.close()
 
@@ -124,7 +124,7 @@ def test_cluster_pair_kernel_and_single_cta_kernel_against_the_oracle(ctx, shape
 @pytest.mark.parametrize("H,KV,hd,T,pre", [(4, 2, 128, 130, 0), (16, 1, 64, 300, 45), (8, 4, 64, 129, 128), (16, 2, 128, 257, 3)],
                          ids=["g2_hd128", "g16_hd64_over_45", "g2_hd64_over_128", "g8_hd128_over_3"])
 def test_cluster_pair_kernel_group_sizes_and_ragged_edges(ctx, H, KV, hd, T, pre):
-    """Group sizes 2, 8 and 16 at both head dims (the pair kernel at 128, the one-CTA kernel at 64), row counts one past
+    """Group sizes 2, 8 and 16 at both head dims, row counts one past
     a tile, and existing cache lengths that leave the first step ragged."""
     import shainet_b200 as S
     rng = np.random.default_rng(3011)
