@@ -76,3 +76,49 @@ def test_batched_tokens_of_an_odd_group_size(ctx):
             same = np.array_equal(o.export_cache()[0], g.cache.export()[0])
             assert rel_err(got[b:b + 1], ref) <= (DECODE_TOL if fmt == "f32" or same else 5e-3), (fmt, b)
             g.close()
+
+
+@pytest.mark.parametrize("T", [2, 5, 40, 63])
+@pytest.mark.parametrize("hd,fmt", [(64, "f32"), (128, "f32"), (64, "bf16"), (128, "bf16")])
+def test_non_finite_rows_of_later_tokens_do_not_reach_earlier_ones(ctx, hd, fmt, T):
+    """A drafted token whose V or K row holds an infinity or NaN: the tokens before it are bit for bit what they are with
+    finite rows in its place."""
+    rng = np.random.default_rng(hd + T)
+    shape = dict(H=8, KV=2, hd=hd, theta=10000.0)
+    for L in (0, 61, 700):
+        kc, vc = (rng.standard_normal((2, L, hd), dtype=np.float32) for _ in range(2))
+        q, k, v = qkv(rng, shape, T)
+        outs = []
+        bad = T // 2   # the first bad token
+        for value in (1.0, np.inf, np.nan):
+            _, g = make_pair(ctx, shape, rng, kv_format=fmt)
+            if L:
+                g.cache.import_(kc, vc)
+            vb, kb = v.copy(), k.copy()
+            vb[bad:, 3::hd] = value
+            if value != 1.0:
+                kb[T - 1] = np.nan
+            outs.append(g.forward_cached(q, kb, vb))
+            g.close()
+        for out in outs[1:]:
+            assert np.array_equal(out[:bad], outs[0][:bad]), (L, np.isnan(out[:bad]).sum())
+            assert not np.isfinite(out[bad:].reshape(T - bad, 8, hd)[:, :, 3]).any()
+
+
+@pytest.mark.parametrize("hd,fmt", [(64, "f32"), (128, "bf16")])
+def test_an_infinite_cached_column_stays_infinite(ctx, hd, fmt):
+    """Every cached V row holds +Inf in one column: so does every output, also where a short last tile of positions lies
+    where an earlier tile lay."""
+    rng = np.random.default_rng(hd)
+    shape = dict(H=16, KV=16, hd=hd, theta=10000.0)
+    for L, T in ((130, 2), (9001, 40)):
+        kc, vc = (rng.standard_normal((16, L, hd), dtype=np.float32) for _ in range(2))
+        vc[:, :, 3] = np.inf
+        q, k, v = qkv(rng, shape, T)
+        v[:, 3::hd] = np.inf
+        _, g = make_pair(ctx, shape, rng, kv_format=fmt)
+        g.cache.import_(kc, vc)
+        out = g.forward_cached(q, k, v).reshape(T, 16, hd)
+        assert (out[:, :, 3] == np.inf).all()
+        assert np.isfinite(np.delete(out, 3, axis=2)).all()
+        g.close()
