@@ -421,13 +421,11 @@ int run_step(shainet_attn_ctx* ctx, const shainet_attn_kv* par, SeqRef seqs, int
         if (par->es != 4 && kern != Kernel::Rows) {
             // These attention kernels read fp32 rows.  A bfloat16 cache is widened (exactly) into
             // a scratch image first; the capacity of the image is a whole number of the
-            // tensor-core kernel's 128-row tiles, and it never holds anything but finite values.
+            // tensor-core kernel's 128-row tiles, whose rows behind max_visible are zeros.
             const int cap_s = (max_visible + 127) / 128 * 128;
             const size_t per = (size_t)hs.num_kv_heads * cap_s * hs.head_dim;
-            float* before = ctx->kv_f32.p;
             rc = grow(ctx->kv_f32, 2 * per, s);
             if (rc) return rc;
-            if (ctx->kv_f32.p != before) CU(cudaMemsetAsync(ctx->kv_f32.p, 0, ctx->kv_f32.cap * sizeof(float), s));
             float* wk = ctx->kv_f32.p;
             float* wv = wk + per;
             CU(launch_kv_widen(seqs.one.k, seqs.one.v, seqs.one.capacity, wk, wv, cap_s, hs.num_kv_heads, hs.head_dim, seqs.one.start,

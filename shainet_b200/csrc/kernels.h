@@ -177,12 +177,13 @@ cudaError_t launch_gather_wait(const unsigned long long* words, float* data, lon
 cudaError_t launch_fill_normal(float* base, int num_kv_heads, int capacity, int head_dim, int len,
                                unsigned long long seed, int elem_bytes, cudaStream_t s);
 
-// Rows [row0, row0 + rows) of every kv head copied between two caches of possibly different
-// element sizes (4 = fp32, 2 = bfloat16; fp32 -> bfloat16 rounds to nearest even) and capacities.
 // Rows [0, rows) of a bfloat16 cache's K and V as fp32 [kv_heads, dst_capacity, head_dim]; the kernel ahead in the stream may
-// still be writing the rows from `start` on, and nothing that reads wk or wv may still run once it does.
+// still be writing the rows from `start` on, and nothing that reads wk or wv may still run once it does.  Rows [rows,
+// dst_capacity) are set to zero where head_dim is a multiple of 8 (the only reader beyond `rows` is the tensor-core kernel).
 cudaError_t launch_kv_widen(const void* k, const void* v, int src_capacity, float* wk, float* wv, int dst_capacity, int num_kv_heads,
                             int head_dim, int start, int rows, cudaStream_t s);
+// Rows [row0, row0 + rows) of every kv head copied between two caches of possibly different
+// element sizes (4 = fp32, 2 = bfloat16; fp32 -> bfloat16 rounds to nearest even) and capacities.
 cudaError_t launch_kv_convert(const void* src, int src_elem_bytes, int src_capacity, void* dst, int dst_elem_bytes,
                               int dst_capacity, int num_kv_heads, int head_dim, int row0, int rows, cudaStream_t s);
 

@@ -404,10 +404,12 @@ __global__ void kv_convert_kernel(const void* src, int src_es, long long src_pit
 
 // Rows [0, rows) of a bfloat16 cache widened into the fp32 image, K and V in one launch: eight elements per load, four loads in
 // flight per thread.  The kernel ahead in the stream appends the rows from `start` on; the older ones, nearly all of
-// them, are widened while it still runs.
+// them, are widened while it still runs.  The image's rows behind them (up to its whole last position tile) are set to zero:
+// the tensor-core kernels load them and multiply them by zero probabilities, and what an earlier call left there need not
+// be finite.
 constexpr int WIDEN_VECS = 4;
 __global__ void __launch_bounds__(256) kv_widen_kernel(const uint4* k, const uint4* v, float4* wk, float4* wv, long long src_pitch,
-                                                       long long dst_pitch, long long old_vecs, long long vecs) {
+                                                       long long dst_pitch, long long old_vecs, long long vecs) {   // dst_pitch: vectors of a head's image, too
     const uint4* src = (blockIdx.z ? v : k) + blockIdx.y * src_pitch;
     float4* dst = (blockIdx.z ? wv : wk) + 2 * blockIdx.y * dst_pitch;
     const long long i0 = (long long)blockIdx.x * (256 * WIDEN_VECS);
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(256) kv_widen_kernel(const uint4* k, const uin
 #pragma unroll
     for (int u = 0; u < WIDEN_VECS; ++u) {
         const long long i = i0 + u * 256 + threadIdx.x;
-        if (i < vecs) {   // a bfloat16 is the upper half of the fp32 of the same value
+        if (i < dst_pitch) {   // a bfloat16 is the upper half of the fp32 of the same value
             dst[2 * i] = make_float4(__uint_as_float(w[u].x << 16), __uint_as_float(w[u].x & 0xffff0000u), __uint_as_float(w[u].y << 16),
                                      __uint_as_float(w[u].y & 0xffff0000u));
             dst[2 * i + 1] = make_float4(__uint_as_float(w[u].z << 16), __uint_as_float(w[u].z & 0xffff0000u),
@@ -441,7 +443,7 @@ cudaError_t launch_kv_widen(const void* k, const void* v, int src_capacity, floa
     }
     const long long per_row = head_dim / 8, vecs = per_row * rows;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)((vecs + 256 * WIDEN_VECS - 1) / (256 * WIDEN_VECS)), num_kv_heads, 2);
+    cfg.gridDim = dim3((unsigned)((per_row * dst_capacity + 256 * WIDEN_VECS - 1) / (256 * WIDEN_VECS)), num_kv_heads, 2);
     cfg.blockDim = dim3(256);
     cfg.stream = s;
     cudaLaunchAttribute at[1];

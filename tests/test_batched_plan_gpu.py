@@ -68,3 +68,22 @@ def test_widened_bf16_cache(ctx, hd, pre, T):
         same = np.array_equal(o.export_cache()[0], g.cache.export()[0])
         assert rel_err(got, ref) <= (2e-3 if n >= 64 and hd >= 64 else DECODE_TOL if same else 5e-3), rel_err(got, ref)
     g.close()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_widened_image_holds_nothing_of_an_earlier_cache(ctx, hd):
+    """The fp32 image ends on a whole position tile: what a longer cache with infinities left there does not reach a shorter
+    one, whose masked positions the tensor cores multiply by zero probabilities."""
+    shape = dict(H=4, KV=2, hd=hd, theta=10000.0)
+    rng = np.random.default_rng(hd)
+    _, a = make_pair(ctx, shape, rng, kv_format="bf16")
+    q, k, v = qkv(rng, shape, 128)
+    v[:, ::2] = np.inf
+    a.forward_cached(q, k, v)
+    o, b = make_pair(ctx, shape, rng, kv_format="bf16")
+    q, k, v = qkv(rng, shape, 70)
+    ref = o.attend_cached(q, k, v, threads=4)
+    got = b.forward_cached(q, k, v)
+    assert rel_err(got, ref) <= 2e-3, rel_err(got, ref)   # TF32 operands
+    a.close()
+    b.close()
