@@ -176,11 +176,34 @@ int gemm_tc(shainet_attn_ctx* ctx, const Q8Maps* w0, const Q8Maps* w1, int M, in
     return SHAINET_ATTN_OK;
 }
 
-// Before the planes and the partials are written on stream s: the newest q8_gemv_dev call on another stream has used them.
+// Before a call's first use of the planes, the partials and the gate|up products on stream s: the newest call that used them, if it
+// was on another stream, comes first.
 int planes_acquire(shainet_attn_ctx* ctx, cudaStream_t s) {
-    if (ctx->planes_pending && ctx->planes_stream != s) CU(cudaStreamWaitEvent(s, ctx->planes_ev, 0));
+    if (ctx->planes_in_use) return SHAINET_ATTN_OK;
+    if (ctx->planes_pending) {
+        unsigned long long id = 0;
+        CU(cudaStreamGetId(s, &id));
+        if (id != ctx->planes_stream) CU(cudaStreamWaitEvent(s, ctx->planes_ev, 0));
+    }
+    ctx->planes_in_use = true;
     return SHAINET_ATTN_OK;
 }
+
+// One entry call that may use them: however it ends, what it has enqueued is recorded as the newest use.
+struct PlanesUse {
+    shainet_attn_ctx* ctx;
+    cudaStream_t s;
+    ~PlanesUse() {
+        if (!ctx->planes_in_use) return;
+        ctx->planes_in_use = false;
+        ctx->planes_pending = (ctx->planes_ev || cudaEventCreateWithFlags(&ctx->planes_ev, cudaEventDisableTiming) == cudaSuccess) &&
+                              cudaEventRecord(ctx->planes_ev, s) == cudaSuccess && cudaStreamGetId(s, &ctx->planes_stream) == cudaSuccess;
+        if (!ctx->planes_pending) {
+            cudaStreamSynchronize(s);
+            cudaGetLastError();
+        }
+    }
+};
 
 // Rows x [M, K] (RMS-normalised with gamma unless it is null) as the planes gemm_tc reads.
 int make_planes(shainet_attn_ctx* ctx, const float* x, int M, int K, const float* gamma, double eps, cudaStream_t s) {
@@ -215,11 +238,11 @@ bool block_tensor_path(const shainet_attn_block* b, int T) {
 int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T, cudaStream_t s) {
     shainet_attn_ctx* ctx = b->ctx;
     const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
-    int rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
+    int rc = planes_acquire(ctx, s);
+    if (!rc) rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
     if (!rc) rc = grow(ctx->act[ACT_ATTN], (size_t)T * qd, s);
     if (!rc && b->gate) rc = grow(ctx->act[ACT_H], (size_t)T * d, s);
     if (!rc && b->gate) rc = grow(ctx->gate_up, (size_t)T * 2 * b->ffn, s);
-    if (!rc) rc = planes_acquire(ctx, s);
     if (!rc) rc = grow(ctx->planes, planes_floats(T, std::max(std::max(d, qd), b->ffn)), s);
     if (rc) return rc;
     float* qbuf = ctx->act[ACT_QKV].p;
@@ -416,16 +439,12 @@ int shainet_attn_q8_gemv_dev(shainet_attn_ctx* ctx, const shainet_attn_q8* w, co
     DeviceGuard g(ctx->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     if (M > 1 && !few_rows(M, w->K) && w->maps.ok && w->K <= MAX_PLANE_K && aligned16(x_dev)) {
+        PlanesUse use{ctx, s};
         int rc = planes_acquire(ctx, s);
         if (!rc) rc = grow(ctx->planes, planes_floats(M, w->K), s);
         if (!rc) rc = make_planes(ctx, x_dev, M, w->K, nullptr, 0.0, s);
         if (!rc) rc = gemm_tc(ctx, &w->maps, nullptr, M, w->K, rows_out(y_dev, w->N, nullptr), nullptr, s);
-        if (rc) return rc;
-        if (!ctx->planes_ev) CU(cudaEventCreateWithFlags(&ctx->planes_ev, cudaEventDisableTiming));
-        CU(cudaEventRecord(ctx->planes_ev, s));
-        ctx->planes_stream = s;
-        ctx->planes_pending = true;
-        return SHAINET_ATTN_OK;
+        return rc;
     }
     return gemv(ctx, x_dev, w->q, w->scales, nullptr, nullptr, y_dev, M, w->N, w->K, nullptr, 0.0, nullptr, nullptr, nullptr, s);
 }
@@ -527,7 +546,9 @@ int shainet_attn_block_forward_dev(shainet_attn_ctx* ctx, shainet_attn_block* b,
     if (new_tokens == 0) return SHAINET_ATTN_OK;
     if (!x_dev || !out_dev || !aligned16(x_dev) || !aligned16(out_dev)) return fail(SHAINET_ATTN_E_INVALID, "null or misaligned tensor pointer");
     DeviceGuard g(ctx->device);
-    return block_forward(b, x_dev, out_dev, new_tokens, stream ? (cudaStream_t)stream : ctx->stream);
+    cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
+    PlanesUse use{ctx, s};
+    return block_forward(b, x_dev, out_dev, new_tokens, s);
 }
 
 int shainet_attn_block_forward_host(shainet_attn_ctx* ctx, shainet_attn_block* b, const float* x, float* out, int new_tokens) {
@@ -537,6 +558,7 @@ int shainet_attn_block_forward_host(shainet_attn_ctx* ctx, shainet_attn_block* b
     if (!x || !out) return fail(SHAINET_ATTN_E_INVALID, "null tensor pointer");
     DeviceGuard g(ctx->device);
     cudaStream_t s = ctx->stream;
+    PlanesUse use{ctx, s};
     const size_t n = (size_t)new_tokens * b->d_model;
     int rc = grow(ctx->dev_in, n, s);
     if (!rc) rc = grow(ctx->dev_out, n, s);
@@ -604,6 +626,7 @@ int shainet_attn_decoder_run(shainet_attn_ctx* ctx, shainet_attn_decoder* dec, c
     if (n_tokens <= 0 || !token_ids) return fail(SHAINET_ATTN_E_INVALID, "no token ids");
     DeviceGuard g(ctx->device);
     cudaStream_t s = ctx->stream;
+    PlanesUse use{ctx, s};
     int rc = decoder_reserve_ids(dec, n_tokens);
     if (rc) return rc;
     memcpy(dec->ids_pin, token_ids, sizeof(int) * (size_t)n_tokens);
@@ -621,6 +644,7 @@ int shainet_attn_decoder_generate(shainet_attn_ctx* ctx, shainet_attn_decoder* d
     if (n_prompt <= 0 || !prompt_ids || steps <= 0 || !tokens_host) return fail(SHAINET_ATTN_E_INVALID, "no prompt, no steps or no output array");
     DeviceGuard g(ctx->device);
     cudaStream_t s = ctx->stream;
+    PlanesUse use{ctx, s};
     int rc = decoder_reserve_ids(dec, n_prompt);
     if (rc) return rc;
     if (dec->history_cap < steps) {

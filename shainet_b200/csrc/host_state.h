@@ -30,10 +30,12 @@ struct shainet_attn_ctx {
     shainet::DevBuf q_rot, part, part_words, dev_in, dev_out;
     shainet::DevBuf kv_f32;             // fp32 image of a bfloat16 cache's rows, for the kernels that read fp32 caches only
     shainet::DevBuf planes, gemm_part, gate_up;   // row scales and planes, split-K partials and raw gate|up products of the tensor-core projections
-    // q8_gemv_dev may be called on any stream: the newest such use of these buffers, which a use on another stream waits for
-    cudaStream_t planes_stream = nullptr;
+    // Calls on any stream use these three buffers: the newest call that did, which one on another stream waits for (streams are
+    // told apart by their id, a handle may be a later stream's), and whether the call under way does
+    unsigned long long planes_stream = 0;
     cudaEvent_t planes_ev = nullptr;
     bool planes_pending = false;
+    bool planes_in_use = false;
     shainet::DevBuf act[6];             // activations of the block / decoder entries (see decoder.cu)   // part_words: {value, epoch} partials of single-sequence decode
     float* pin_in = nullptr;
     size_t pin_in_cap = 0;

@@ -82,3 +82,68 @@ def test_error_is_that_of_fp32_sums(ctx, K, M):
         assert err <= {2048: 1.15e-7, 8192: 1.33e-7}[K] * (1.0 if len(rows) > 1 else 1.2), (rows[0], err)
     assert (got[3] == 0).all() and not np.isfinite(got[4]).any() and np.isnan(got[5]).all()
     W.close()
+
+
+def test_products_on_two_streams_keep_to_themselves(ctx):
+    """The scratch of a context's products is shared by calls on different streams: other activations, weights and outputs
+    on each of them, back and forth, long enough to overlap."""
+    import torch
+    import shainet_b200 as S
+    rng = np.random.default_rng(8)
+    dev = torch.device("cuda:0")
+    K, N, M = 2048, 4096, 1500
+    jobs = []
+    for i in range(2):
+        q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+        s = (0.001 * (0.5 + rng.random((N, K // 32)))).astype(np.float32)
+        x = rng.standard_normal((M - 700 * i, K)).astype(np.float32)
+        W = S.Q8Weight.from_quantized(ctx, q, s)
+        w = torch.from_numpy(q).to(dev).double() * torch.from_numpy(s).to(dev).double().repeat_interleave(32, 1)
+        tx = torch.from_numpy(x).to(dev)
+        jobs.append((W, tx, [torch.full((len(x), N), float("nan"), device=dev) for _ in range(6)], (tx.double() @ w.T).cpu().numpy(), torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    for r in range(6):
+        for W, tx, ys, _, st in jobs:
+            W.gemv_dev(tx.data_ptr(), ys[r].data_ptr(), len(tx), st.cuda_stream)
+    torch.cuda.synchronize()
+    ctx.sync()
+    for W, _, ys, truth, _ in jobs:
+        for y in ys:
+            assert rel_err(y.cpu().numpy(), truth) <= DECODE_TOL
+        W.close()
+
+
+def test_a_block_and_products_on_other_streams(ctx):
+    """A block of several tokens on one stream and products on two others use the same scratch: block, product, block,
+    product without a synchronisation between them give what they give one by one."""
+    import torch
+    import shainet_b200 as S
+    from test_q8_decoder_gpu import _make_block
+    rng = np.random.default_rng(81)
+    d, T, K, N, M = 2048, 300, 2048, 8192, 900
+    _, block, owned = _make_block(ctx, rng, d, 32, 8, 64, 8192, 5e5, 1e-5, False)
+    q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+    s = (0.001 * (0.5 + rng.random((N, K // 32)))).astype(np.float32)
+    W = S.Q8Weight.from_quantized(ctx, q, s)
+    xb, xw = torch.randn(3, T, d, device="cuda"), torch.randn(3, M, K, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    results = []
+    for one_by_one in (True, False):
+        block.clear_cache()
+        yb, yw = torch.full_like(xb, float("nan")), torch.full((3, M, N), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        for r in range(3):   # the block always on the first stream: its cache grows in order
+            block.forward_cached_dev(xb[r].data_ptr(), yb[r].data_ptr(), T, streams[0].cuda_stream)
+            if one_by_one:
+                torch.cuda.synchronize()
+            W.gemv_dev(xw[r].data_ptr(), yw[r].data_ptr(), M, streams[1 + r % 2].cuda_stream)
+            if one_by_one:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        ctx.sync()
+        results.append((yb, yw))
+    assert torch.isfinite(results[0][0]).all() and torch.isfinite(results[0][1]).all()
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    W.close()
+    for o in owned:
+        o.close()
