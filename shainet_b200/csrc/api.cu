@@ -645,7 +645,7 @@ int shainet_attn_ctx_destroy(shainet_attn_ctx* c) {
     if (c->live_caches != 0) return fail(SHAINET_ATTN_E_STATE, "%d caches still alive", c->live_caches);
     DeviceGuard g(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (DevBuf* b : {&c->q_rot, &c->part, &c->part_words, &c->dev_in, &c->dev_out, &c->kv_f32, &c->planes, &c->gemm_part, &c->gate_up})
+    for (DevBuf* b : {&c->q_rot, &c->part, &c->part_words, &c->dev_in, &c->dev_out, &c->kv_f32, &c->planes, &c->gemm_part})
         if (b->p) cudaFree(b->p);
     for (DevBuf& b : c->act)
         if (b.p) cudaFree(b.p);
@@ -705,7 +705,7 @@ int shainet_attn_ctx_timing_read(shainet_attn_ctx* c, double* total_ms, int* lau
 size_t shainet_attn_ctx_scratch_bytes(shainet_attn_ctx* c) {
     if (!c) return 0;
     return (c->q_rot.cap + c->part.cap + c->part_words.cap + c->dev_in.cap + c->dev_out.cap + c->kv_f32.cap + c->planes.cap +
-            c->gemm_part.cap + c->gate_up.cap) * sizeof(float);
+            c->gemm_part.cap) * sizeof(float);
 }
 
 int shainet_attn_kv_create(shainet_attn_ctx* ctx, shainet_attn_kv** out, int num_heads, int num_kv_heads,

@@ -176,8 +176,8 @@ int gemm_tc(shainet_attn_ctx* ctx, const Q8Maps* w0, const Q8Maps* w1, int M, in
     return SHAINET_ATTN_OK;
 }
 
-// Before a call's first use of the planes, the partials and the gate|up products on stream s: the newest call that used them, if it
-// was on another stream, comes first.
+// Before a call's first use of the planes and the partials on stream s: the newest call that used them, if it was on another
+// stream, comes first.
 int planes_acquire(shainet_attn_ctx* ctx, cudaStream_t s) {
     if (ctx->planes_in_use) return SHAINET_ATTN_OK;
     if (ctx->planes_pending) {
@@ -187,6 +187,17 @@ int planes_acquire(shainet_attn_ctx* ctx, cudaStream_t s) {
     }
     ctx->planes_in_use = true;
     return SHAINET_ATTN_OK;
+}
+
+// A stream that is being captured (or cannot tell: launches on it then fail as they do).  The shared scratch is neither grown nor
+// ordered against what a graph's replays do, so captured calls keep to the kernels that need none of it.
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
 }
 
 // One entry call that may use them: however it ends, what it has enqueued is recorded as the newest use.
@@ -242,7 +253,7 @@ int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T,
     if (!rc) rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
     if (!rc) rc = grow(ctx->act[ACT_ATTN], (size_t)T * qd, s);
     if (!rc && b->gate) rc = grow(ctx->act[ACT_H], (size_t)T * d, s);
-    if (!rc && b->gate) rc = grow(ctx->gate_up, (size_t)T * 2 * b->ffn, s);
+    if (!rc && b->gate) rc = grow(ctx->act[ACT_HIDDEN], (size_t)T * 2 * b->ffn, s);   // the raw gate|up products
     if (!rc) rc = grow(ctx->planes, planes_floats(T, std::max(std::max(d, qd), b->ffn)), s);
     if (rc) return rc;
     float* qbuf = ctx->act[ACT_QKV].p;
@@ -275,16 +286,16 @@ int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T,
     r.M = T;
     r.K = d;
     CU(launch_q8_rows(r, s));
-    rc = gemm_tc(ctx, &b->gate->maps, &b->up->maps, T, d, rows_out(ctx->gate_up.p, 2 * b->ffn, nullptr), &splits, s);
+    rc = gemm_tc(ctx, &b->gate->maps, &b->up->maps, T, d, rows_out(ctx->act[ACT_HIDDEN].p, 2 * b->ffn, nullptr), &splits, s);
     if (rc) return rc;
-    CU(launch_q8_swiglu(splits > 1 ? ctx->gemm_part.p : ctx->gate_up.p, splits, (size_t)T * 2 * b->ffn, T, b->ffn,
+    CU(launch_q8_swiglu(splits > 1 ? ctx->gemm_part.p : ctx->act[ACT_HIDDEN].p, splits, (size_t)T * 2 * b->ffn, T, b->ffn,
                         planes_of(ctx, T), ctx->planes.p, ctx->sm_count, s));
     return gemm_tc(ctx, &b->down->maps, nullptr, T, b->ffn, rows_out(out, d, h), nullptr, s);
 }
 
 // LlamaBlock#forward_cached (llama_block.cr:189-196) on device pointers.
 int block_forward(shainet_attn_block* b, const float* x, float* out, int T, cudaStream_t s) {
-    if (T > 1 && block_tensor_path(b, T)) return block_forward_rows(b, x, out, T, s);
+    if (T > 1 && block_tensor_path(b, T) && !capturing(s)) return block_forward_rows(b, x, out, T, s);
     shainet_attn_ctx* ctx = b->ctx;
     const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
     int rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
@@ -438,7 +449,7 @@ int shainet_attn_q8_gemv_dev(shainet_attn_ctx* ctx, const shainet_attn_q8* w, co
     if (M < 0) return fail(SHAINET_ATTN_E_INVALID, "negative row count");
     DeviceGuard g(ctx->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    if (M > 1 && !few_rows(M, w->K) && w->maps.ok && w->K <= MAX_PLANE_K && aligned16(x_dev)) {
+    if (M > 1 && !few_rows(M, w->K) && w->maps.ok && w->K <= MAX_PLANE_K && aligned16(x_dev) && !capturing(s)) {
         PlanesUse use{ctx, s};
         int rc = planes_acquire(ctx, s);
         if (!rc) rc = grow(ctx->planes, planes_floats(M, w->K), s);

@@ -147,3 +147,70 @@ def test_a_block_and_products_on_other_streams(ctx):
     W.close()
     for o in owned:
         o.close()
+
+
+@pytest.mark.parametrize("K,N,M", [(2048, 512, 6), (2048, 512, 200), (1536, 300, 40)], ids=lambda v: str(v))
+def test_several_rows_under_stream_capture(ctx, K, N, M):
+    """A captured product of several rows replays with new activations, on a context that has made no such product before
+    and whatever is called beside the graph."""
+    import torch
+    import shainet_b200 as S
+    rng = np.random.default_rng(K + N + M)
+    q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+    s = (0.001 * (0.5 + rng.random((N, K // 32)))).astype(np.float32)
+    w = q.astype(np.float64) * s.astype(np.float64).repeat(32, 1)
+    c = S.AttnContext(0)
+    W = S.Q8Weight.from_quantized(c, q, s)
+    tx, ty = torch.empty((M, K), device="cuda"), torch.empty((M, N), device="cuda")
+    other = torch.empty((M, N), device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        W.gemv_dev(tx.data_ptr(), ty.data_ptr(), M, torch.cuda.current_stream().cuda_stream)
+    for _ in range(2):
+        x = rng.standard_normal((M, K)).astype(np.float32)
+        tx.copy_(torch.from_numpy(x))
+        torch.cuda.synchronize()
+        graph.replay()
+        W.gemv_dev(tx.data_ptr(), other.data_ptr(), M)   # on the context's stream, beside the replay
+        torch.cuda.synchronize()
+        c.sync()
+        truth = x.astype(np.float64) @ w.T
+        assert rel_err(ty.cpu().numpy(), truth) <= DECODE_TOL
+        assert rel_err(other.cpu().numpy(), truth) <= DECODE_TOL
+    del graph
+    W.close()
+    c.close()
+
+
+def test_a_block_of_several_tokens_under_stream_capture(ctx):
+    """After one plain call with as many tokens a captured block call finds all its scratch; its replay is the plain call's
+    result to the block's tolerance (other kernels)."""
+    import torch
+    import shainet_b200 as S
+    from test_q8_decoder_gpu import BLOCK_TOL, _make_block
+    rng = np.random.default_rng(82)
+    d, T = 2048, 9
+    c = S.AttnContext(0)
+    _, block, owned = _make_block(c, rng, d, 32, 8, 64, 4096, 5e5, 1e-5, False)
+    x, y, z = (torch.randn(T, d, device="cuda") for _ in range(3))
+    torch.cuda.synchronize()
+    block.forward_cached_dev(x.data_ptr(), y.data_ptr(), T)
+    c.sync()
+    block.clear_cache()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        block.forward_cached_dev(x.data_ptr(), z.data_ptr(), T, torch.cuda.current_stream().cuda_stream)
+    for seed in range(2):
+        x.copy_(torch.randn(T, d, device="cuda"))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        block.clear_cache()
+        block.forward_cached_dev(x.data_ptr(), y.data_ptr(), T)
+        c.sync()
+        assert rel_err(z.cpu().numpy(), y.cpu().numpy()) <= BLOCK_TOL
+    del graph
+    for o in owned:
+        o.close()
+    c.close()
