@@ -245,57 +245,103 @@ bool block_tensor_path(const shainet_attn_block* b, int T) {
     return b->qkv_maps.ok && b->wo->maps.ok && (!b->gate || (b->gate->maps.ok && b->up->maps.ok && b->down->maps.ok));
 }
 
-// Several new tokens: the projections on the tensor cores.
-int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T, cudaStream_t s) {
+// o_proj, residual and FFN of n tokens whose attention rows are at `attn`.
+int block_ffn_rows(shainet_attn_block* b, const float* x, const float* attn, float* out, int n, cudaStream_t s) {
     shainet_attn_ctx* ctx = b->ctx;
-    const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
-    int rc = planes_acquire(ctx, s);
-    if (!rc) rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
-    if (!rc) rc = grow(ctx->act[ACT_ATTN], (size_t)T * qd, s);
-    if (!rc && b->gate) rc = grow(ctx->act[ACT_H], (size_t)T * d, s);
-    if (!rc && b->gate) rc = grow(ctx->act[ACT_HIDDEN], (size_t)T * 2 * b->ffn, s);   // the raw gate|up products
-    if (!rc) rc = grow(ctx->planes, planes_floats(T, std::max(std::max(d, qd), b->ffn)), s);
+    const int d = b->d_model, qd = b->q_dim;
+    int rc = make_planes(ctx, attn, n, qd, nullptr, 0.0, s);
     if (rc) return rc;
-    float* qbuf = ctx->act[ACT_QKV].p;
-    float* kbuf = qbuf + (size_t)T * qd;
-    float* vbuf = kbuf + (size_t)T * kd;
-    rc = make_planes(ctx, x, T, d, b->norm1, b->eps, s);
-    if (rc) return rc;
-    const Q8GemmOut qkv{{qbuf, kbuf, vbuf}, {0, qd, qd + kd}, {qd, kd, kd}, 3, 0, nullptr};
-    rc = gemm_tc(ctx, &b->qkv_maps, nullptr, T, d, qkv, nullptr, s);
-    if (rc) return rc;
-    float* attn = ctx->act[ACT_ATTN].p;
-    rc = forward_device(ctx, b->kv, qbuf, kbuf, vbuf, attn, T, b->scale, 0, s);
-    if (!rc) rc = make_planes(ctx, attn, T, qd, nullptr, 0.0, s);
-    if (rc) return rc;
-    if (!b->gate) return gemm_tc(ctx, &b->wo->maps, nullptr, T, qd, rows_out(out, d, x), nullptr, s);
+    if (!b->gate) return gemm_tc(ctx, &b->wo->maps, nullptr, n, qd, rows_out(out, d, x), nullptr, s);
     float* h = ctx->act[ACT_H].p;
     int splits = 1;
-    rc = gemm_tc(ctx, &b->wo->maps, nullptr, T, qd, rows_out(h, d, x), &splits, s);
+    rc = gemm_tc(ctx, &b->wo->maps, nullptr, n, qd, rows_out(h, d, x), &splits, s);
     if (rc) return rc;
     Q8RowsArgs r{};   // h = x + o_proj, its norm and its planes in one pass
     r.x = splits > 1 ? ctx->gemm_part.p : h;
     r.splits = splits > 1 ? splits : 0;
-    r.split_stride = (size_t)T * d;
+    r.split_stride = (size_t)n * d;
     r.residual = x;
     r.h = h;
     r.gamma = b->norm2;
     r.eps = b->eps;
-    r.planes = planes_of(ctx, T);
+    r.planes = planes_of(ctx, n);
     r.row_scale = ctx->planes.p;
-    r.M = T;
+    r.M = n;
     r.K = d;
     CU(launch_q8_rows(r, s));
-    rc = gemm_tc(ctx, &b->gate->maps, &b->up->maps, T, d, rows_out(ctx->act[ACT_HIDDEN].p, 2 * b->ffn, nullptr), &splits, s);
+    rc = gemm_tc(ctx, &b->gate->maps, &b->up->maps, n, d, rows_out(ctx->act[ACT_HIDDEN].p, 2 * b->ffn, nullptr), &splits, s);
     if (rc) return rc;
-    CU(launch_q8_swiglu(splits > 1 ? ctx->gemm_part.p : ctx->act[ACT_HIDDEN].p, splits, (size_t)T * 2 * b->ffn, T, b->ffn,
-                        planes_of(ctx, T), ctx->planes.p, ctx->sm_count, s));
-    return gemm_tc(ctx, &b->down->maps, nullptr, T, b->ffn, rows_out(out, d, h), nullptr, s);
+    CU(launch_q8_swiglu(splits > 1 ? ctx->gemm_part.p : ctx->act[ACT_HIDDEN].p, splits, (size_t)n * 2 * b->ffn, n, b->ffn,
+                        planes_of(ctx, n), ctx->planes.p, ctx->sm_count, s));
+    return gemm_tc(ctx, &b->down->maps, nullptr, n, b->ffn, rows_out(out, d, h), nullptr, s);
+}
+
+// Tokens of one pass over the projections.  It bounds what a prompt needs beside the row kernels' scratch (raw gate|up products
+// and planes), and is halved where the device has no room for that.  At 8192 tokens of the LLaMA-3.2-1B shape passes of 2048
+// cost 4 %: their last waves of tiles are emptier.
+constexpr int PASS_TOKENS = 8192, MIN_PASS_TOKENS = 256;
+
+// Scratch of passes of up to n rows through products of K inputs and n0 + n1 outputs.
+size_t split_floats(const shainet_attn_ctx* ctx, int n, int K, int n0, int n1) {
+    const Q8GemmPlan p = q8_gemm_plan(n, K, n0, n1, ctx->sm_count);
+    return p.splits > 1 ? (size_t)n * (n0 + n1) * p.splits : 0;
+}
+
+// Everything block_forward_rows needs beside the attention call's own scratch; *pass: tokens of a pass that there is room for.
+int block_reserve_rows(shainet_attn_block* b, int T, int* pass, cudaStream_t s) {
+    shainet_attn_ctx* ctx = b->ctx;
+    const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim, ffn = b->ffn;
+    int rc = planes_acquire(ctx, s);
+    if (!rc) rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
+    if (!rc) rc = grow(ctx->act[ACT_ATTN], (size_t)T * qd, s);
+    if (!rc && b->gate) rc = grow(ctx->act[ACT_H], (size_t)T * d, s);
+    if (rc) return rc;
+    for (*pass = std::min(T, PASS_TOKENS);; *pass = std::max(*pass / 2, std::min(T, MIN_PASS_TOKENS))) {
+        size_t part = 0;
+        for (int n : {*pass, T % *pass}) {
+            if (n == 0) continue;
+            part = std::max({part, split_floats(ctx, n, d, qd + 2 * kd, 0), split_floats(ctx, n, qd, d, 0)});
+            if (b->gate) part = std::max({part, split_floats(ctx, n, d, ffn, ffn), split_floats(ctx, n, ffn, d, 0)});
+        }
+        // the raw gate|up products of a pass; a captured call of as many tokens finds its hidden rows there
+        rc = b->gate ? grow(ctx->act[ACT_HIDDEN], std::max((size_t)T, (size_t)2 * *pass) * ffn, s) : SHAINET_ATTN_OK;
+        if (!rc) rc = grow(ctx->planes, planes_floats(*pass, std::max(std::max(d, qd), ffn)), s);
+        if (!rc && part) rc = grow(ctx->gemm_part, part, s);
+        if (rc != SHAINET_ATTN_E_NOMEM || *pass <= MIN_PASS_TOKENS) return rc;
+    }
+}
+
+// Several new tokens: the projections on the tensor cores.
+int block_forward_rows(shainet_attn_block* b, const float* x, float* out, int T, int pass, cudaStream_t s) {
+    shainet_attn_ctx* ctx = b->ctx;
+    const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
+    int rc = SHAINET_ATTN_OK;
+    float* qbuf = ctx->act[ACT_QKV].p;
+    float* kbuf = qbuf + (size_t)T * qd;
+    float* vbuf = kbuf + (size_t)T * kd;
+    for (int t = 0; t < T; t += pass) {
+        const int n = std::min(pass, T - t);
+        rc = make_planes(ctx, x + (size_t)t * d, n, d, b->norm1, b->eps, s);
+        if (rc) return rc;
+        const Q8GemmOut qkv{{qbuf + (size_t)t * qd, kbuf + (size_t)t * kd, vbuf + (size_t)t * kd}, {0, qd, qd + kd}, {qd, kd, kd}, 3, 0, nullptr};
+        rc = gemm_tc(ctx, &b->qkv_maps, nullptr, n, d, qkv, nullptr, s);
+        if (rc) return rc;
+    }
+    float* attn = ctx->act[ACT_ATTN].p;
+    rc = forward_device(ctx, b->kv, qbuf, kbuf, vbuf, attn, T, b->scale, 0, s);
+    for (int t = 0; !rc && t < T; t += pass)
+        rc = block_ffn_rows(b, x + (size_t)t * d, attn + (size_t)t * qd, out + (size_t)t * d, std::min(pass, T - t), s);
+    return rc;
 }
 
 // LlamaBlock#forward_cached (llama_block.cr:189-196) on device pointers.
 int block_forward(shainet_attn_block* b, const float* x, float* out, int T, cudaStream_t s) {
-    if (T > 1 && block_tensor_path(b, T) && !capturing(s)) return block_forward_rows(b, x, out, T, s);
+    if (T > 1 && block_tensor_path(b, T) && !capturing(s)) {
+        int pass = 0;
+        const int room = block_reserve_rows(b, T, &pass, s);
+        if (room == SHAINET_ATTN_OK) return block_forward_rows(b, x, out, T, pass, s);
+        if (room != SHAINET_ATTN_E_NOMEM) return room;   // otherwise the kernels that need less
+    }
     shainet_attn_ctx* ctx = b->ctx;
     const int d = b->d_model, qd = b->q_dim, kd = b->kv_dim;
     int rc = grow(ctx->act[ACT_QKV], (size_t)T * (qd + 2 * kd), s);
@@ -451,11 +497,25 @@ int shainet_attn_q8_gemv_dev(shainet_attn_ctx* ctx, const shainet_attn_q8* w, co
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     if (M > 1 && !few_rows(M, w->K) && w->maps.ok && w->K <= MAX_PLANE_K && aligned16(x_dev) && !capturing(s)) {
         PlanesUse use{ctx, s};
-        int rc = planes_acquire(ctx, s);
-        if (!rc) rc = grow(ctx->planes, planes_floats(M, w->K), s);
-        if (!rc) rc = make_planes(ctx, x_dev, M, w->K, nullptr, 0.0, s);
-        if (!rc) rc = gemm_tc(ctx, &w->maps, nullptr, M, w->K, rows_out(y_dev, w->N, nullptr), nullptr, s);
-        return rc;
+        int pass = std::min(M, PASS_TOKENS), rc = planes_acquire(ctx, s);
+        while (!rc) {
+            const int tail = M % pass;
+            const size_t part = std::max(split_floats(ctx, pass, w->K, w->N, 0), tail ? split_floats(ctx, tail, w->K, w->N, 0) : 0);
+            rc = grow(ctx->planes, planes_floats(pass, w->K), s);
+            if (!rc && part) rc = grow(ctx->gemm_part, part, s);
+            if (rc != SHAINET_ATTN_E_NOMEM || pass <= MIN_PASS_TOKENS) break;
+            pass = std::max(pass / 2, MIN_PASS_TOKENS);
+            rc = SHAINET_ATTN_OK;
+        }
+        if (rc && rc != SHAINET_ATTN_E_NOMEM) return rc;
+        if (!rc) {
+            for (int t = 0; !rc && t < M; t += pass) {
+                const int n = std::min(pass, M - t);
+                rc = make_planes(ctx, x_dev + (size_t)t * w->K, n, w->K, nullptr, 0.0, s);
+                if (!rc) rc = gemm_tc(ctx, &w->maps, nullptr, n, w->K, rows_out(y_dev + (size_t)t * w->N, w->N, nullptr), nullptr, s);
+            }
+            return rc;
+        }
     }
     return gemv(ctx, x_dev, w->q, w->scales, nullptr, nullptr, y_dev, M, w->N, w->K, nullptr, 0.0, nullptr, nullptr, nullptr, s);
 }

@@ -214,3 +214,79 @@ def test_a_block_of_several_tokens_under_stream_capture(ctx):
     for o in owned:
         o.close()
     c.close()
+
+
+def test_more_rows_than_one_pass(ctx):
+    """A product and a block of more tokens than a pass takes: the rows of the second pass are those of a call of their own."""
+    import torch
+    import shainet_b200 as S
+    from test_q8_decoder_gpu import _make_block
+    rng = np.random.default_rng(83)
+    K, N, M, P = 256, 300, 8192 + 130, 8192
+    q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+    s = (0.001 * (0.5 + rng.random((N, K // 32)))).astype(np.float32)
+    W = S.Q8Weight.from_quantized(ctx, q, s)
+    x = torch.randn(M, K, device="cuda")
+    y, z = torch.full((M, N), float("nan"), device="cuda"), torch.full((M - P, N), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    W.gemv_dev(x.data_ptr(), y.data_ptr(), M)
+    W.gemv_dev(x[P:].data_ptr(), z.data_ptr(), M - P)
+    ctx.sync()
+    truth = x.cpu().numpy().astype(np.float64) @ (q.astype(np.float64) * s.astype(np.float64).repeat(32, 1)).T
+    assert rel_err(y.cpu().numpy(), truth) <= DECODE_TOL and torch.equal(y[P:], z)
+    W.close()
+    for ffn in (512, 0):
+        _, block, owned = _make_block(ctx, rng, 256, 4, 2, 64, ffn, 5e5, 1e-5, False)
+        x, y = torch.randn(M, 256, device="cuda"), torch.empty(M, 256, device="cuda")
+        z = torch.empty(M - P, 256, device="cuda")
+        torch.cuda.synchronize()
+        block.forward_cached_dev(x.data_ptr(), y.data_ptr(), M)
+        ctx.sync()
+        block.clear_cache()
+        first = torch.empty(P, 256, device="cuda")
+        torch.cuda.synchronize()
+        block.forward_cached_dev(x.data_ptr(), first.data_ptr(), P)
+        block.forward_cached_dev(x[P:].data_ptr(), z.data_ptr(), M - P)
+        block.clear_cache()
+        inplace = x.clone()
+        torch.cuda.synchronize()
+        block.forward_cached_dev(inplace.data_ptr(), inplace.data_ptr(), M)
+        ctx.sync()
+        assert torch.equal(y[:P], first) and torch.equal(y[P:], z) and torch.equal(inplace, y)
+        for o in owned:
+            o.close()
+
+
+@pytest.mark.parametrize("free_mb", [110, 36])
+def test_without_memory_for_the_planes(free_mb):
+    """Where the device has no room for the planes of all rows the product of several rows takes fewer at a time, and the row
+    kernels, which need no scratch, where it has none at all."""
+    import torch
+    import shainet_b200 as S
+    rng = np.random.default_rng(84)
+    K, N, M = 51200, 64, 2048   # planes of 2048 rows: 400 MB and more, of 256 rows: more than 48
+    c = S.AttnContext(0)
+    q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+    s = (0.001 * (0.5 + rng.random((N, K // 32)))).astype(np.float32)
+    W = S.Q8Weight.from_quantized(c, q, s)
+    x = torch.randn(M, K, device="cuda")
+    short, roomy = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    torch.cuda.synchronize()
+    W.gemv_dev(x.data_ptr(), short.data_ptr(), 1)   # loads the row kernel
+    c.sync()
+    assert c.scratch_bytes() < 16 << 20
+    held = []
+    for size in (1 << 30, 1 << 26, 12 << 20):   # down to at most 12 MB more than free_mb
+        while torch.cuda.mem_get_info()[0] > size + (free_mb << 20):
+            held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+    W.gemv_dev(x.data_ptr(), short.data_ptr(), M)
+    c.sync()
+    assert (c.scratch_bytes() < 16 << 20) if free_mb == 36 else ((48 << 20) < c.scratch_bytes() < (122 << 20))
+    del held
+    torch.cuda.empty_cache()
+    W.gemv_dev(x.data_ptr(), roomy.data_ptr(), M)
+    c.sync()
+    assert c.scratch_bytes() >= 400 << 20
+    assert rel_err(short.cpu().numpy(), roomy.cpu().numpy()) <= 2 * DECODE_TOL   # either is within DECODE_TOL of the exact product
+    W.close()
+    c.close()
