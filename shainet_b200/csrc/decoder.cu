@@ -141,21 +141,19 @@ int gemv(shainet_attn_ctx* ctx, const float* x, const signed char* q, const floa
     return SHAINET_ATTN_OK;
 }
 
-// ctx->planes of M rows: their scales (padded, so that the planes behind them are aligned for TMA), then [2][M][K] halves.
-constexpr size_t scale_floats(size_t M) { return (M + 63) / 64 * 64; }
-constexpr size_t planes_floats(size_t M, size_t K) { return scale_floats(M) + M * K; }
-__half* planes_of(shainet_attn_ctx* ctx, int M) { return reinterpret_cast<__half*>(ctx->planes.p + scale_floats(M)); }
-constexpr int MAX_PLANE_K = 50 * 1024;   // a row is held in shared memory while its planes are made
+// ctx->planes of M rows of K activations: [3][M][K] bfloat16.
+constexpr size_t planes_floats(size_t M, size_t K) { return (3 * M * K + 1) / 2; }
+__nv_bfloat16* planes_of(shainet_attn_ctx* ctx) { return reinterpret_cast<__nv_bfloat16*>(ctx->planes.p); }
+constexpr int MAX_PLANE_K = 50 * 1024;   // as for the row kernels; a row is held in shared memory while it is normalised
 
-// Tensor-core product of planes [2][M][K] with one or two weights (their columns beside each other) into `out`.  Where
+// Tensor-core product of planes [3][M][K] with one or two weights (their columns beside each other) into `out`.  Where
 // the plan splits the contraction: the splits are added into `out` (defer == null), or left in ctx->gemm_part
 // [splits][M][N] for the caller, who finds their number in *defer (1: `out` is complete).
 int gemm_tc(shainet_attn_ctx* ctx, const Q8Maps* w0, const Q8Maps* w1, int M, int K, const Q8GemmOut& out, int* defer, cudaStream_t s) {
     const int N = w0->N + (w1 ? w1->N : 0);
     const Q8GemmPlan plan = q8_gemm_plan(M, K, w0->N, w1 ? w1->N : 0, ctx->sm_count);
     Q8GemmArgs g{};
-    g.planes = planes_of(ctx, M);
-    g.row_scale = ctx->planes.p;
+    g.planes = planes_of(ctx);
     g.w[0] = w0;
     g.w[1] = w1;
     g.M = M;
@@ -222,8 +220,7 @@ int make_planes(shainet_attn_ctx* ctx, const float* x, int M, int K, const float
     r.x = x;
     r.gamma = gamma;
     r.eps = eps;
-    r.planes = planes_of(ctx, M);
-    r.row_scale = ctx->planes.p;
+    r.planes = planes_of(ctx);
     r.M = M;
     r.K = K;
     CU(launch_q8_rows(r, s));
@@ -264,15 +261,14 @@ int block_ffn_rows(shainet_attn_block* b, const float* x, const float* attn, flo
     r.h = h;
     r.gamma = b->norm2;
     r.eps = b->eps;
-    r.planes = planes_of(ctx, n);
-    r.row_scale = ctx->planes.p;
+    r.planes = planes_of(ctx);
     r.M = n;
     r.K = d;
     CU(launch_q8_rows(r, s));
     rc = gemm_tc(ctx, &b->gate->maps, &b->up->maps, n, d, rows_out(ctx->act[ACT_HIDDEN].p, 2 * b->ffn, nullptr), &splits, s);
     if (rc) return rc;
     CU(launch_q8_swiglu(splits > 1 ? ctx->gemm_part.p : ctx->act[ACT_HIDDEN].p, splits, (size_t)n * 2 * b->ffn, n, b->ffn,
-                        planes_of(ctx, n), ctx->planes.p, ctx->sm_count, s));
+                        planes_of(ctx), ctx->sm_count, s));
     return gemm_tc(ctx, &b->down->maps, nullptr, n, b->ffn, rows_out(out, d, h), nullptr, s);
 }
 

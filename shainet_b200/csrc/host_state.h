@@ -29,7 +29,7 @@ struct shainet_attn_ctx {
     cudaStream_t stream = nullptr;
     shainet::DevBuf q_rot, part, part_words, dev_in, dev_out;
     shainet::DevBuf kv_f32;             // fp32 image of a bfloat16 cache's rows, for the kernels that read fp32 caches only
-    shainet::DevBuf planes, gemm_part;   // row scales and planes, split-K partials of the tensor-core projections
+    shainet::DevBuf planes, gemm_part;   // bfloat16 planes, split-K partials of the tensor-core projections
     // Calls on any stream use these two buffers: the newest call that did, which one on another stream waits for (streams are
     // told apart by their id, a handle may be a later stream's), and whether the call under way does
     unsigned long long planes_stream = 0;

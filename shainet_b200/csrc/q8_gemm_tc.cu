@@ -5,29 +5,30 @@
 // small kernels around it, the host loops between the projections (rms_norm.cr:18-37, swiglu_ff.cr:76-91,
 // llama_block.cr:189-196), with the single-row kernels' precision:
 //
-//  * the int8 weights are exact in half precision;
-//  * an fp32 activation, its row scaled by a power of two, is the sum of two halves up to 2^-24 of it (split2 below), so two
-//    products per weight reproduce the fp32 product to its own rounding;
+//  * the int8 weights are exact in bfloat16;
+//  * an fp32 activation is exactly the sum of three bfloat16 values (8 + 8 + 8 significand bits: truncate, subtract,
+//    truncate, subtract; below 2^-109 what is lost is less than 2^-133), so three products per weight reproduce the fp32
+//    product with nothing rounded away, whatever else stands in the row;
 //  * the products of one 32-input scale block accumulate in fp32 in tensor memory; a block is then multiplied by its
 //    fp32 scale and added to fp32 accumulators in registers, sixteen blocks at a time by themselves (a single chain over
 //    8192 inputs loses twice as much).
-// Against f64 the error (2-norm) is that of the row kernels: 1.0e-7 at 2048 inputs, 1.2e-7 at 8192.
+// Against f64 the error (2-norm) is 0.9e-7 at 2048 inputs and 1.0e-7 at 8192, that of the row kernels 1.04e-7 and 1.21e-7.
 //
 // A pair of CTAs (cta_group::2) computes 256 weight rows x NT tokens.  The weights are the A operand: raw int8 tiles
-// arrive by TMA, four convert warps (one thread per weight row) turn 32 of them at a time into pairs of halves and put
-// them into tensor memory; the activations are the B operand, two planes of halves prepared by a kernel ahead, each CTA
+// arrive by TMA, four convert warps (one thread per weight row) turn 32 of them at a time into pairs of bfloat16 and put
+// them into tensor memory; the activations are the B operand, three bfloat16 planes prepared by a kernel ahead, each CTA
 // loading its half of the tokens.  Lanes of tensor memory are weight rows, so a thread of the accumulating warps needs
 // one scale per block and stores its outputs coalesced over the lanes.
 //
 // Bounds.  The tensor core multiplies 4096 pairs per cycle and SM, but an MMA of 16 inputs takes at least about 64
-// cycles, however few its columns (the 128 rows of A have to pass).  At 128 tokens the two planes are two passes: 256
-// cycles per 32-input block; what a block takes is 700, the hand-overs between convert, MMA and accumulating warps over the
-// three accumulators that tensor memory has room for.  With up to 64 tokens the planes lie side by side as 2 NT columns
-// of one pass, and the accumulating warps add the two columns of a token; the launch is then bound by the convert warps
-// and the contraction is split over the pairs (split-K) until they are all busy.
-// Measured, planes and split sums included: 4096 x 2048 -> 16384 in 737 us (three bfloat16 planes and eight accumulating
-// warps 761 us, and an error of 1.5e-7; row tiles of four on the CUDA cores 20.7 ms), 64 x 2048 -> 8192 in 28 us (186 us).
-#include <cuda_fp16.h>
+// cycles, however few its columns (the 128 rows of A have to pass).  At 128 tokens the three planes are three passes: 384
+// cycles per 32-input block, 0.2 us; what a block takes is 0.43 us, the hand-overs between convert, MMA and accumulating warps
+// over the three accumulators that tensor memory has room for.  At 64 tokens there is room for six.  With up to 32 tokens the planes lie
+// side by side as 3 NT columns of one pass, and the accumulating warps add the three columns of a token; the launch is then
+// bound by the convert warps and the contraction is split over the pairs (split-K) until they are all busy.
+// Measured, planes and split sums included: 4096 x 2048 -> 16384 in 777 us (row tiles of four on the CUDA cores 20.7 ms),
+// 64 x 2048 -> 8192 in 22 us (186 us).
+#include <cuda_bf16.h>
 #include <math.h>
 #include <algorithm>
 #include <atomic>
@@ -63,9 +64,9 @@ __device__ __forceinline__ f32x2 qt_fma(f32x2 a, f32x2 b, f32x2 c) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Instruction descriptor: fp32 accumulate, half-precision A and B (both K-major), dense.
-__host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
-    return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// Instruction descriptor: fp32 accumulate, bfloat16 A and B (both K-major), dense.
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // NT tokens per tile (128, 64, 32 or 16).
@@ -73,16 +74,16 @@ template <int NT_>
 struct QT {
     static constexpr int NT = NT_;
     static constexpr int ROWS = 128;                     // weight rows per CTA, 256 per pair
-    static constexpr bool STACK = NT <= 64;              // the planes are columns of one pass, not two passes
-    static constexpr int D_COLS = STACK ? 2 * NT : NT;   // columns of one block accumulator
-    static constexpr int ND = NT == 16 ? 8 : NT == 32 ? 6 : 3;   // block accumulators (and A slots) in tensor memory
-    static constexpr int A_COLS = 16;                    // 32 halves per lane
+    static constexpr bool STACK = NT <= 32;              // the planes are columns of one pass, not three passes
+    static constexpr int D_COLS = STACK ? 3 * NT : NT;   // columns of one block accumulator
+    static constexpr int ND = NT == 16 ? 8 : NT == 32 ? 4 : NT == 64 ? 6 : 3;   // block accumulators (and A slots) in tensor memory
+    static constexpr int A_COLS = 16;                    // 32 bfloat16 per lane
     static constexpr int TMEM_A = ND * D_COLS;
     static constexpr int TMEM_COLS = 512;
     static constexpr int NB = 6;                         // B stages of 64 inputs
-    static constexpr int PLANE_BYTES = (NT / 2) * 128;   // this CTA's half of the tokens, 64 halves each
-    static constexpr int B_BYTES = 2 * PLANE_BYTES;
-    static constexpr int NW = 6;                         // raw weight stages of 128 inputs
+    static constexpr int PLANE_BYTES = (NT / 2) * 128;   // this CTA's half of the tokens, 64 bfloat16 each
+    static constexpr int B_BYTES = 3 * PLANE_BYTES;
+    static constexpr int NW = NT == 128 ? 3 : 6;         // raw weight stages of 128 inputs
     static constexpr int W_BYTES = ROWS * 128;
     static constexpr int NS = 8;                         // scale stages of 4 blocks
     static constexpr int S_BYTES = ROWS * 16;
@@ -150,13 +151,13 @@ struct QtArgs {
     int t_tiles;
     int splits;
     Q8GemmOut out;
-    const float* row_scale;   // [M]: the power of two that undoes the token's scaling
     AttnStatus* status;
 };
 
-// Where both planes share an accumulator the last MMA of a block cuts its fp32 result towards zero: on average by
-// 2^-24 / (2 ln 2) of it, the mean of half an ulp over the value (measured 4.1e-8).  That is put back as a gain in the
-// last sum, before it is rounded; what stays has zero mean.
+// Where the planes share an accumulator the last MMA of a block cuts its fp32 result towards zero: on average by
+// 2^-24 / (2 ln 2) of it, the mean of half an ulp over the value (measured 4.3e-8).  That is put back as a gain in the
+// last sum, before it is rounded; what stays has zero mean.  Side by side the planes' sums are not cut: the first one's products
+// have 15 bits, and the fp32 adds of the others round.
 constexpr float TRUNCATED = 0.7213f * 5.9604645e-8f;
 
 template <int NT>
@@ -167,7 +168,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     using C = QT<NT>;
     constexpr int ND = C::ND, NB = C::NB, NW = C::NW, NS = C::NS, CW = C::CW;
     extern __shared__ __align__(1024) unsigned char qt_smem[];
-    unsigned char* b_s = qt_smem;                        // [NB][2 planes][NT/2 tokens][128 bytes], 128-byte swizzle
+    unsigned char* b_s = qt_smem;                        // [NB][3 planes][NT/2 tokens][128 bytes], 128-byte swizzle
     unsigned char* w_s = b_s + NB * C::B_BYTES;          // [NW][128 rows][128 bytes], 128-byte swizzle
     unsigned char* s_s = w_s + NW * C::W_BYTES;          // [NS][128 rows][4 scales]
     uint64_t* bars = reinterpret_cast<uint64_t*>(s_s + NS * C::S_BYTES);
@@ -240,7 +241,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         // ---------------- accumulate: one weight row and CW tokens per thread ----------------
         const int quad = warp & 3, cq = (warp - 8) >> 2;
         const int r = quad * 32 + lane;
-        const uint32_t d_addr = tmem + ((uint32_t)(quad * 32) << 16) + cq * (C::STACK ? 2 * CW : CW);
+        const uint32_t d_addr = tmem + ((uint32_t)(quad * 32) << 16) + cq * (C::STACK ? 3 * CW : CW);
         const uint32_t d_leader = map_to_cta(smem_u32(&d_free[0]), 0u);
         pdl_wait();   // the residual comes from the kernels ahead
         RingPos<NS> rs;
@@ -274,13 +275,16 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                         uint32_t v[C::HC];
                         tmem_ld<C::HC>(da + h, v);
                         if constexpr (C::STACK) {
-                            uint32_t low[C::HC];
-                            tmem_ld<C::HC>(da + CW + h, low);
+                            uint32_t v1[C::HC], v2[C::HC];
+                            tmem_ld<C::HC>(da + CW + h, v1);
+                            tmem_ld<C::HC>(da + 2 * CW + h, v2);
                             tmem_wait_ld();
                             if (h + C::HC == CW) handed_back();
 #pragma unroll
-                            for (int c = 0; c < C::HC; c += 2)
-                                grp[(h + c) / 2] = qt_fma(qt_add(qt_pack_bits(low[c], low[c + 1]), qt_pack_bits(v[c], v[c + 1])), s2, grp[(h + c) / 2]);
+                            for (int c = 0; c < C::HC; c += 2) {
+                                const f32x2 low = qt_add(qt_pack_bits(v2[c], v2[c + 1]), qt_pack_bits(v1[c], v1[c + 1]));
+                                grp[(h + c) / 2] = qt_fma(qt_add(low, qt_pack_bits(v[c], v[c + 1])), s2, grp[(h + c) / 2]);
+                            }
                         } else {
                             tmem_wait_ld();
                             if (h + C::HC == CW) handed_back();
@@ -312,18 +316,17 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                 const int t0 = it.t0 + cq * CW;
 #pragma unroll
                 for (int c0 = 0; c0 < CW; c0 += 4) {   // the loads of four tokens together, then their stores
-                    float ex[4], res[4];
+                    float res[4];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const int t = t0 + c0 + c;
-                        ex[c] = t < a.M ? __ldcg(a.row_scale + t) : 0.0f;
                         res[c] = (a.out.residual != nullptr && t < a.M) ? __ldcg(a.out.residual + (size_t)t * pitch + col) : 0.0f;
                     }
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         float lo, hi;
                         asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[(c0 + c) / 2]));
-                        float v = ((c & 1) ? hi : lo) * ex[c];
+                        float v = (c & 1) ? hi : lo;
                         if (a.out.residual != nullptr) v = __fadd_rn(res[c], v);
                         if (t0 + c0 + c < a.M) dst[(size_t)(t0 + c0 + c) * pitch] = v;
                     }
@@ -347,7 +350,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                         if (leader) mbar_arrive_expect_tx(&b_full[st], 2 * C::B_BYTES);
                         const uint32_t bar = map_to_cta(smem_u32(&b_full[st]), 0u);
 #pragma unroll
-                        for (int p = 0; p < 2; ++p)
+                        for (int p = 0; p < 3; ++p)
                             tma_load_2d_pair(b_s + st * C::B_BYTES + p * C::PLANE_BYTES, &tm_x, g * 64,
                                              p * a.M + it.t0 + (int)rank * (NT / 2), bar);
                     }
@@ -378,7 +381,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         } else if (warp == 1) {
             // ---------------- MMA issuer: one warp of the leader, for both CTAs ----------------
             if (leader) {
-                constexpr uint32_t idesc = idesc_f16(2 * C::ROWS, C::D_COLS);
+                constexpr uint32_t idesc = idesc_bf16(2 * C::ROWS, C::D_COLS);
                 uint32_t stages = 0;      // of all this pair's items: the last ones are not handed back (nobody waits for them)
                 for (int w = pair; w < items; w += pairs) {
                     const Item it = item_of(w);
@@ -399,12 +402,12 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                         const uint32_t d = tmem + rd.slot * C::D_COLS;
                         const uint32_t aw = tmem + C::TMEM_A + rd.slot * C::A_COLS;
                         if (elect_one()) {
-                            constexpr int PASSES = C::STACK ? 1 : 2;
+                            constexpr int PASSES = C::STACK ? 1 : 3;
 #pragma unroll
                             for (int p = PASSES - 1; p >= 0; --p)   // smallest plane first
 #pragma unroll
                                 for (int kk = 0; kk < 2; ++kk)
-                                    mma_ts_f16_pair(d, aw + kk * 8, bd + (uint64_t)((p * C::PLANE_BYTES + half * 64 + kk * 32) >> 4),
+                                    mma_ts_bf16_pair(d, aw + kk * 8, bd + (uint64_t)((p * C::PLANE_BYTES + half * 64 + kk * 32) >> 4),
                                                      idesc, (p < PASSES - 1 || kk > 0) ? 1u : 0u);
                             if (half == 1 && s + NB < stages) tc_commit_both(&b_free[rb.slot]);
                             tc_commit_both(&d_full[rd.slot]);
@@ -417,7 +420,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                 }
             }
         } else if (warp >= 4 && warp < 8) {
-            // ---------------- convert: int8 -> pairs of halves in tensor memory, one weight row per thread ----------------
+            // ---------------- convert: int8 -> pairs of bfloat16 in tensor memory, one weight row per thread ----------------
             const int quad = warp & 3;
             const int r = quad * 32 + lane;
             const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
@@ -440,11 +443,11 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                         }
                         const uint32_t words[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
                         uint32_t out[16];
-                        // b + 128 in the significand of a half of 1024 .. 2047, minus 1152: exact
+                        // the low seven bits in the significand of a bfloat16 of 128 .. 255, minus 128 or, with the sign bit, 256: exact
 #pragma unroll
                         for (int k = 0; k < 16; ++k) {
-                            const uint32_t u = __byte_perm(words[k >> 1] ^ 0x80808080u, 0x64646464u, (k & 1) ? 0x4342 : 0x4140);
-                            asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(out[k]) : "r"(u), "r"(0x64806480u));
+                            const uint32_t u = __byte_perm(words[k >> 1], 0x43434343u, (k & 1) ? 0x4342 : 0x4140);
+                            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(out[k]) : "r"(u & 0xff7fff7fu), "r"(u & 0xff80ff80u));
                         }
                         if (!first_round && !(ok = mbar_wait(&d_full[rd.slot], rd.parity ^ 1u, a.status, 78))) break;
                         tc_fence_after();
@@ -470,82 +473,48 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     }
 }
 
-// A token's scaling: the power of two that brings the largest finite magnitude of its row into [2^14, 2^15) (as two
-// factors, each of which a float holds), and its inverse.
-struct RowScale {
-    float up0, up1, down;
-};
-__device__ __forceinline__ float pow2f(int e) {   // 2^e, e >= -149
-    return e >= -126 ? __uint_as_float((uint32_t)(e + 127) << 23) : __uint_as_float(1u << (e + 149));
-}
-__device__ __forceinline__ RowScale row_scale(float amax) {
-    if (!(amax > 0.0f)) return RowScale{1.0f, 1.0f, 1.0f};
-    const uint32_t b = __float_as_uint(amax);
-    const int e = (b >> 23) ? (int)(b >> 23) - 127 : -118 - __clz(b);   // floor(log2 amax), subnormals included
-    const int up = min(14 - e, 140);                                    // from -113; 2^-140 is still a float, and subnormals are exact there
-    const int h = up >> 1;
-    return RowScale{pow2f(h), pow2f(up - h), pow2f(-up)};
-}
-__device__ __forceinline__ float finite_abs(float x) {
-    const float v = fabsf(x);
-    return v < INFINITY ? v : 0.0f;   // NaN compares false
-}
-__device__ __forceinline__ float finite_abs(const float4& v) {
-    return fmaxf(fmaxf(finite_abs(v.x), finite_abs(v.y)), fmaxf(finite_abs(v.z), finite_abs(v.w)));
+// x as three bfloat16 whose sum is x exactly (Inf and NaN stay in the first).
+__device__ __forceinline__ void split3(float x, unsigned short (&p)[3]) {
+    uint32_t b = __float_as_uint(x);
+    if ((b & 0x7f800000u) == 0x7f800000u) {
+        p[0] = (unsigned short)((b & 0x007fffffu) ? 0x7fc0u : (b >> 16));
+        p[1] = p[2] = 0;
+        return;
+    }
+    const float hi = __uint_as_float(b & 0xffff0000u);
+    const float r1 = __fsub_rn(x, hi);
+    const uint32_t b1 = __float_as_uint(r1);
+    const float r2 = __fsub_rn(r1, __uint_as_float(b1 & 0xffff0000u));
+    p[0] = (unsigned short)(b >> 16);
+    p[1] = (unsigned short)(b1 >> 16);
+    p[2] = (unsigned short)(__float_as_uint(r2) >> 16);
 }
 
-// A scaled activation as two halves.  The first is rounded to nearest, to eleven significant bits and never finer than 1/4 (the
-// row's largest is at least 2^14): its products with int8 weights are multiples of 1/4, and as long as the sum of a 32-input
-// block stays below 2^22 the tensor core, which cuts off what does not fit its 24 bits, adds them without any error (a block
-// of normal deviates is of the order of 2^20).  The second holds the rest to eleven bits: what is left out is at most 2^-24 of
-// x (or 2^-29 of the row's largest).  Infinities and NaN stay in the first.
-__device__ __forceinline__ void split2(float x, const RowScale& r, unsigned short (&p)[2]) {
-    constexpr float GRID = 3145728.0f;   // 1.5 x 2^21: a float there is a multiple of 1/4
-    x = x * r.up0 * r.up1;
-    const __half hi = __float2half_rn(__fsub_rn(__fadd_rn(x, GRID), GRID));
-    const float hf = __half2float(hi);
-    p[0] = __half_as_ushort(hi);
-    p[1] = fabsf(hf) < INFINITY ? __half_as_ushort(__float2half_rn(__fsub_rn(x, hf))) : (unsigned short)0;
-}
-
-__device__ __forceinline__ void store_planes(__half* planes, size_t plane_elems, size_t at, const float4& v, const RowScale& r) {
-    unsigned short p[4][2];
-    split2(v.x, r, p[0]);
-    split2(v.y, r, p[1]);
-    split2(v.z, r, p[2]);
-    split2(v.w, r, p[3]);
+__device__ __forceinline__ void store_planes(__nv_bfloat16* planes, size_t plane_elems, size_t at, const float4& v) {
+    unsigned short p[4][3];
+    split3(v.x, p[0]);
+    split3(v.y, p[1]);
+    split3(v.z, p[2]);
+    split3(v.w, p[3]);
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 3; ++k)
         *reinterpret_cast<uint2*>(planes + k * plane_elems + at) =
             make_uint2((uint32_t)p[0][k] | (uint32_t)p[1][k] << 16, (uint32_t)p[2][k] | (uint32_t)p[3][k] << 16);
 }
 
 constexpr int ROW_THREADS = 256;
 
-__device__ __forceinline__ float block_max(float v, float* red) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float m = red[0];
-#pragma unroll
-    for (int w = 1; w < ROW_THREADS / 32; ++w) m = fmaxf(m, red[w]);
-    return m;
-}
-
-// One CTA per token row: [sum of the splits of the projection ahead + residual -> h], RMSNorm, planes and scale.
-// Memory-bound (4 bytes read and 4 written per element beside the partials); the row stays in shared memory.
+// One CTA per token row: [sum of the splits of the projection ahead + residual -> h], RMSNorm, bfloat16 planes.
+// Memory-bound (4 bytes read, 6 written per element beside the partials).
 __global__ void __launch_bounds__(ROW_THREADS) q8_rows_kernel(Q8RowsArgs a) {
-    extern __shared__ __align__(16) float4 row_s[];   // [K], each element only touched by its thread
+    extern __shared__ __align__(16) float4 row_s[];   // the row, when it is needed twice (norm)
     __shared__ double red[ROW_THREADS / 32];
-    __shared__ float redm[ROW_THREADS / 32];
     const int m = blockIdx.x, n4 = a.K >> 2;
     const size_t base = (size_t)m * a.K;
     const float4* gam = reinterpret_cast<const float4*>(a.gamma);
     pdl_wait();
     pdl_launch_dependents();
     double sq = 0.0;
-    float amax = 0.0f;
     for (int d = threadIdx.x; d < n4; d += ROW_THREADS) {
         float4 v = __ldcg(reinterpret_cast<const float4*>(a.x + base) + d);
         if (a.splits > 0) {
@@ -559,59 +528,49 @@ __global__ void __launch_bounds__(ROW_THREADS) q8_rows_kernel(Q8RowsArgs a) {
             }
             if (a.h != nullptr) reinterpret_cast<float4*>(a.h + base)[d] = v;
         }
-        row_s[d] = v;
-        if (a.gamma == nullptr) amax = fmaxf(amax, finite_abs(v));
-        else sq += (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z + (double)v.w * (double)v.w;
-    }
-    if (a.gamma != nullptr) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
-        __syncthreads();
-        double tot = 0.0;
-#pragma unroll
-        for (int w = 0; w < ROW_THREADS / 32; ++w) tot += red[w];
-        // rms_norm.cr:29-32, as the single-row kernels do it: f64 sum, scaling and weight, one rounding to fp32
-        const double inv_rms = rsqrt(tot / (double)a.K + a.eps);
-        for (int d = threadIdx.x; d < n4; d += ROW_THREADS) {
-            float4 v = row_s[d];
-            const float4 g = __ldg(gam + d);
-            v.x = (float)(((double)v.x * inv_rms) * (double)g.x);
-            v.y = (float)(((double)v.y * inv_rms) * (double)g.y);
-            v.z = (float)(((double)v.z * inv_rms) * (double)g.z);
-            v.w = (float)(((double)v.w * inv_rms) * (double)g.w);
+        if (a.gamma == nullptr) {
+            store_planes(a.planes, (size_t)a.M * a.K, base + 4 * d, v);
+        } else {
             row_s[d] = v;
-            amax = fmaxf(amax, finite_abs(v));
+            sq += (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z + (double)v.w * (double)v.w;
         }
     }
-    const RowScale r = row_scale(block_max(amax, redm));
-    if (threadIdx.x == 0) a.row_scale[m] = r.down;
-    for (int d = threadIdx.x; d < n4; d += ROW_THREADS) store_planes(a.planes, (size_t)a.M * a.K, base + 4 * d, row_s[d], r);
+    if (a.gamma == nullptr) return;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    double tot = 0.0;
+#pragma unroll
+    for (int w = 0; w < ROW_THREADS / 32; ++w) tot += red[w];
+    // rms_norm.cr:29-32, as the single-row kernels do it: f64 sum, scaling and weight, one rounding to fp32
+    const double inv_rms = rsqrt(tot / (double)a.K + a.eps);
+    for (int d = threadIdx.x; d < n4; d += ROW_THREADS) {
+        float4 v = row_s[d];
+        const float4 g = __ldg(gam + d);
+        v.x = (float)(((double)v.x * inv_rms) * (double)g.x);
+        v.y = (float)(((double)v.y * inv_rms) * (double)g.y);
+        v.z = (float)(((double)v.z * inv_rms) * (double)g.z);
+        v.w = (float)(((double)v.w * inv_rms) * (double)g.w);
+        store_planes(a.planes, (size_t)a.M * a.K, base + 4 * d, v);
+    }
 }
 
-// hidden = silu(gate) * up in f64 (swiglu_ff.cr:83-88), rounded to fp32 once, as planes.  `gu`: [splits][M][2 ffn].  A
-// cluster of CTAs per token row: the row's largest magnitude passes through distributed shared memory, so that a few
-// rows still use many SMs (the f64 exponentials of one row of 8192 are 4 us of one SM).
-__global__ void __launch_bounds__(ROW_THREADS) q8_swiglu_kernel(const float* gu, int splits, size_t split_stride, int M, int ffn,
-                                                                __half* planes, float* scales) {
-    extern __shared__ __align__(16) float4 row_s[];   // this CTA's share of the row
-    __shared__ float redm[ROW_THREADS / 32];
-    __shared__ float cta_max;
-    uint32_t ctas;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
-    const uint32_t rank = cluster_ctarank();
-    const size_t m = blockIdx.x / ctas;
-    const int n4 = ffn >> 2, per = (n4 + (int)ctas - 1) / (int)ctas;
-    const int d0 = min(n4, (int)rank * per), d1 = min(n4, d0 + per);
+// hidden = silu(gate) * up in f64 (swiglu_ff.cr:83-88), rounded to fp32 once, as planes.  `gu`: [splits][M][2 ffn].  `parts` CTAs
+// per token row, so that a few rows still use many SMs.  Bound by the f64 exponentials.
+__global__ void __launch_bounds__(ROW_THREADS) q8_swiglu_kernel(const float* gu, int splits, size_t split_stride, int M, int ffn, int parts,
+                                                                __nv_bfloat16* planes) {
+    const int m = blockIdx.x / parts, part = blockIdx.x - m * parts;
+    const int n4 = ffn >> 2, per = (n4 + parts - 1) / parts;
+    const int d0 = min(n4, part * per), d1 = min(n4, d0 + per);
     pdl_wait();
     pdl_launch_dependents();
     auto act = [](float gf, float uf) {
         const double gd = (double)gf;
         return (float)((gd / (1.0 + exp(-gd))) * (double)uf);
     };
-    float amax = 0.0f;
     for (int d = d0 + threadIdx.x; d < d1; d += ROW_THREADS) {
-        const float* g = gu + m * 2 * ffn + 4 * d;
+        const float* g = gu + (size_t)m * 2 * ffn + 4 * d;
         float4 gv = __ldcg(reinterpret_cast<const float4*>(g)), uv = __ldcg(reinterpret_cast<const float4*>(g + ffn));
         for (int z = 1; z < splits; ++z) {
             const float4 p = __ldcg(reinterpret_cast<const float4*>(g + z * split_stride));
@@ -619,24 +578,9 @@ __global__ void __launch_bounds__(ROW_THREADS) q8_swiglu_kernel(const float* gu,
             gv = make_float4(gv.x + p.x, gv.y + p.y, gv.z + p.z, gv.w + p.w);
             uv = make_float4(uv.x + q.x, uv.y + q.y, uv.z + q.z, uv.w + q.w);
         }
-        const float4 v = make_float4(act(gv.x, uv.x), act(gv.y, uv.y), act(gv.z, uv.z), act(gv.w, uv.w));
-        row_s[d - d0] = v;
-        amax = fmaxf(amax, finite_abs(v));
+        store_planes(planes, (size_t)M * ffn, (size_t)m * ffn + 4 * d,
+                     make_float4(act(gv.x, uv.x), act(gv.y, uv.y), act(gv.z, uv.z), act(gv.w, uv.w)));
     }
-    amax = block_max(amax, redm);
-    if (ctas > 1) {
-        if (threadIdx.x == 0) cta_max = amax;
-        cluster_sync_all();
-        for (uint32_t c = 0; c < ctas; ++c) {
-            float v;
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(&cta_max), c)));
-            amax = fmaxf(amax, v);
-        }
-        cluster_sync_all();   // nobody leaves while its maximum may still be read
-    }
-    const RowScale r = row_scale(amax);
-    if (threadIdx.x == 0 && rank == 0) scales[m] = r.down;
-    for (int d = d0 + threadIdx.x; d < d1; d += ROW_THREADS) store_planes(planes, (size_t)M * ffn, m * ffn + 4 * d, row_s[d - d0], r);
 }
 
 // Sum of the splits into the (up to three) outputs of a launch without a norm behind it.
@@ -753,10 +697,9 @@ cudaError_t launch_q8_gemm_tc(const Q8GemmArgs& g, const Q8GemmPlan& plan, int s
     a.t_tiles = (g.M + plan.nt - 1) / plan.nt;
     a.splits = plan.splits;
     a.out = g.out;
-    a.row_scale = g.row_scale;
     a.status = g.status;
     CUtensorMap tx;
-    if (!make_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.planes, g.K, 2ull * g.M, 2ull * g.K, 64, plan.nt / 2, CU_TENSOR_MAP_SWIZZLE_128B))
+    if (!make_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, g.planes, g.K, 3ull * g.M, 2ull * g.K, 64, plan.nt / 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
     const long long items = (long long)a.n_tiles * a.t_tiles * a.splits;
     if (items > 0x7fffffff) return cudaErrorInvalidValue;
@@ -773,7 +716,7 @@ cudaError_t launch_q8_gemm_tc(const Q8GemmArgs& g, const Q8GemmPlan& plan, int s
 cudaError_t launch_q8_rows(const Q8RowsArgs& a, cudaStream_t s) {
     if (a.M <= 0) return cudaSuccess;
     if (a.K % 4 != 0) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)a.K * 4;
+    const size_t smem = a.gamma ? (size_t)a.K * 4 : 0;   // the row is needed twice
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     if (smem > 40 * 1024) {
         static std::atomic<unsigned long long> configured{0};
@@ -783,21 +726,12 @@ cudaError_t launch_q8_rows(const Q8RowsArgs& a, cudaStream_t s) {
     return launch_chain(q8_rows_kernel, dim3(a.M), ROW_THREADS, smem, 1, s, a);
 }
 
-cudaError_t launch_q8_swiglu(const float* gu, int splits, size_t split_stride, int M, int ffn, __half* planes, float* row_scale, int sm_count,
-                             cudaStream_t s) {
+cudaError_t launch_q8_swiglu(const float* gu, int splits, size_t split_stride, int M, int ffn, __nv_bfloat16* planes, int sm_count, cudaStream_t s) {
     if (M <= 0) return cudaSuccess;
     if (ffn % 4 != 0) return cudaErrorInvalidValue;
-    int ctas = 1;   // per row: as many as it takes to give every SM two
-    while (ctas < 8 && (long long)M * ctas < 2ll * sm_count) ctas *= 2;
-    const size_t smem = (size_t)((ffn / 4 + ctas - 1) / ctas) * 16;
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    if (smem > 40 * 1024) {
-        static std::atomic<unsigned long long> configured{0};
-        cudaError_t e = allow_smem(q8_swiglu_kernel, 200 * 1024, configured);
-        if (e != cudaSuccess) return e;
-    }
-    return launch_chain(q8_swiglu_kernel, dim3((unsigned)(M * ctas)), ROW_THREADS, smem, ctas, s, gu, splits, split_stride, M, ffn, planes,
-                        row_scale);
+    int parts = 1;   // as many as it takes to give every SM two CTAs
+    while (parts < 8 && (long long)M * parts < 2ll * sm_count) parts *= 2;
+    return launch_chain(q8_swiglu_kernel, dim3((unsigned)(M * parts)), ROW_THREADS, 0, 1, s, gu, splits, split_stride, M, ffn, parts, planes);
 }
 
 cudaError_t launch_q8_reduce(const float* part, int splits, size_t split_stride, int M, int N, const Q8GemmOut& out, cudaStream_t s) {

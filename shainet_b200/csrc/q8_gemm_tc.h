@@ -1,7 +1,7 @@
 // Launch interface of the tensor-core Q8_0 matrix product (several activation rows) and of the row kernels around it.
 #pragma once
 #include <cuda.h>
-#include <cuda_fp16.h>
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -29,8 +29,7 @@ struct Q8GemmOut {
 };
 
 struct Q8GemmArgs {
-    const __half* planes;          // [2][M][K], token t scaled by a power of two
-    const float* row_scale;        // [M], its inverse
+    const __nv_bfloat16* planes;   // [3][M][K]
     const Q8Maps* w[2];            // the second (nullable) weight's columns follow the first's
     int M, K;
     Q8GemmOut out;
@@ -45,7 +44,7 @@ Q8GemmPlan q8_gemm_plan(int M, int K, int n0, int n1, int sm_count);
 cudaError_t launch_q8_gemm_tc(const Q8GemmArgs& g, const Q8GemmPlan& plan, int sm_count, cudaStream_t s);
 
 // One token row after another: splits == 0: row = x; otherwise row = residual + sum over splits of x, also stored to h.
-// Then RMSNorm with gamma (nullable) and the split into two planes of halves [2][M][K] with their scales [M].  K up to 51200.
+// Then RMSNorm with gamma (nullable; K up to 51200) and the split into three bfloat16 planes [3][M][K].
 struct Q8RowsArgs {
     const float* x;
     int splits;
@@ -54,14 +53,12 @@ struct Q8RowsArgs {
     float* h;                // nullable
     const float* gamma;      // nullable
     double eps;
-    __half* planes;
-    float* row_scale;
+    __nv_bfloat16* planes;
     int M, K;
 };
 cudaError_t launch_q8_rows(const Q8RowsArgs& a, cudaStream_t s);
 // planes of silu(gate) * up; gu is [splits][M][2 * ffn], gate columns first.
-cudaError_t launch_q8_swiglu(const float* gu, int splits, size_t split_stride, int M, int ffn, __half* planes, float* row_scale, int sm_count,
-                             cudaStream_t s);
+cudaError_t launch_q8_swiglu(const float* gu, int splits, size_t split_stride, int M, int ffn, __nv_bfloat16* planes, int sm_count, cudaStream_t s);
 // Sum of the splits [splits][M][N] into `out`.
 cudaError_t launch_q8_reduce(const float* part, int splits, size_t split_stride, int M, int N, const Q8GemmOut& out, cudaStream_t s);
 

@@ -1,8 +1,8 @@
 """Q8_0 products with several activation rows on the tensor cores, against an f64 product with the dequantised weight.
 
-Tolerance: int8 weights are exact halves, an fp32 activation is the sum of two halves up to 2^-24 of it (or 2^-29 of its row's
-largest), what else is left are fp32 sums of K <= 8192 terms; with the error normalised by the largest output, sqrt(K) 2^-24
-times a few for the tensor core's truncating adds stays below 1e-5, the tolerance of the single-row kernels."""
+Tolerance: the products are exact (int8 weights are bfloat16 values, an fp32 activation is the sum of three of them), what
+is left are fp32 sums of K <= 8192 terms; with the error normalised by the largest output, sqrt(K) 2^-24 times a few for
+the tensor core's truncating adds stays below 1e-5, the tolerance of the single-row kernels."""
 import numpy as np
 import pytest
 
@@ -290,3 +290,29 @@ def test_without_memory_for_the_planes(free_mb):
     assert rel_err(short.cpu().numpy(), roomy.cpu().numpy()) <= 2 * DECODE_TOL   # either is within DECODE_TOL of the exact product
     W.close()
     c.close()
+
+
+@pytest.mark.parametrize("M", [16, 64, 200])
+@pytest.mark.parametrize("outlier", [1e4, 1e6])
+def test_small_activations_beside_a_large_one(ctx, outlier, M):
+    """One channel 10^4 or 10^6 times the others, with zero weights: the outputs are those of the others, to the error of
+    the row kernels (2-norm; 1.04e-7 with a tenth of room)."""
+    import torch
+    import shainet_b200 as S
+    rng = np.random.default_rng(M)
+    K, N = 2048, 512
+    q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+    q[:, 77] = 0
+    s = (0.001 * rng.random((N, K // 32))).astype(np.float32)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    x[:, 77] *= np.float32(outlier)
+    W = S.Q8Weight.from_quantized(ctx, q, s)
+    tx = torch.from_numpy(x).cuda()
+    ty = torch.empty((M, N), device="cuda")
+    torch.cuda.synchronize()
+    W.gemv_dev(tx.data_ptr(), ty.data_ptr(), M)
+    ctx.sync()
+    truth = x.astype(np.float64) @ (q.astype(np.float64) * s.astype(np.float64).repeat(32, 1)).T
+    err = np.linalg.norm(ty.cpu().numpy() - truth) / np.linalg.norm(truth)
+    assert err <= 1.15e-7, err
+    W.close()
