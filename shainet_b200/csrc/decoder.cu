@@ -232,9 +232,11 @@ Q8GemmOut rows_out(float* y, int N, const float* residual) { return Q8GemmOut{{y
 
 enum { ACT_QKV = 0, ACT_ATTN = 1, ACT_H = 2, ACT_HIDDEN = 3, ACT_A = 4, ACT_B = 5 };
 
-// Up to four rows the single-row kernels' row tiles read the weights once, in one launch (2048 -> 8192: 11 us for two rows
-// and 16 us for four, against 18 us for planes, product and split sum); they need whole 2048-input segments.
-bool few_rows(int M, int K) { return M <= 4 && q8_fast_path(K); }
+// Two rows, and three or four while one row tile holds them, stay with the row kernels: one launch that reads the weights once (or
+// twice: two rows of more than 20480 inputs), against planes, product and split sum.  Row kernels and tensor path, us: 2048 -> 8192
+// 11 (two rows) and 16 (four) against 18; 10240 -> 4096 34 (four); in two tiles 12288 -> 4096 44 (three) and 47 (four) against 36;
+// 24576 -> 2048 in tiles of one 30 (two), 41 (three) and 51 (four) against 39.
+bool few_rows(int M, int K) { return q8_fast_path(K) && (M <= 2 || (M <= 4 && q8_row_tile(M, K) >= M)); }
 
 bool block_tensor_path(const shainet_attn_block* b, int T) {
     if (std::max(std::max(b->d_model, b->q_dim), b->gate ? b->ffn : 0) > MAX_PLANE_K) return false;

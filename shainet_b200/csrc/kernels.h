@@ -208,6 +208,7 @@ struct Q8GemvArgs {
     int M, N, K;
 };
 bool q8_fast_path(int K);
+int q8_row_tile(int M, int K);   // rows (4, 2 or 1) of M that the row kernels take per pass over the weights, as shared memory allows
 cudaError_t launch_q8_gemv(const Q8GemvArgs& a, int sm_count, cudaStream_t s);
 // x[t] = table[ids[t]] for `rows` tokens; also zeroes n_words arg-max words.
 cudaError_t launch_embed_rows(const int* ids_dev, const float* table, float* x, int rows, int d_model, int vocab,

@@ -782,6 +782,12 @@ cudaError_t launch_fast(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
 
 bool q8_fast_path(int K) { return K > 0 && K % 128 == 0 && (size_t)padded_k(K) * sizeof(float) <= 200 * 1024; }
 
+int q8_row_tile(int M, int K) {
+    for (int rows : {4, 2})
+        if (M > rows / 2 && (size_t)rows * padded_k(K) * sizeof(float) <= 160 * 1024) return rows;
+    return 1;
+}
+
 cudaError_t launch_q8_gemv(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;
     if (a.K <= 0) return cudaErrorInvalidValue;
@@ -789,17 +795,12 @@ cudaError_t launch_q8_gemv(const Q8GemvArgs& a, int sm_count, cudaStream_t s) {
     if (q8_fast_path(a.K) && (reinterpret_cast<uintptr_t>(a.q) & 15u) == 0 && (!swiglu || (reinterpret_cast<uintptr_t>(a.q2) & 15u) == 0) &&
         (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0 && (a.gamma == nullptr || (reinterpret_cast<uintptr_t>(a.gamma) & 15u) == 0)) {
         if (ring_ok(a, sm_count)) return swiglu ? launch_ring<RG_NS, true>(a, sm_count, s) : launch_ring<RG_NS, false>(a, sm_count, s);
-        // Rows are taken four at a time while that fits shared memory; a row tile re-reads the weights.
-        const bool four = a.M >= 3 && (size_t)4 * padded_k(a.K) * sizeof(float) <= 160 * 1024;
-        const bool two = !four && a.M >= 2 && (size_t)2 * padded_k(a.K) * sizeof(float) <= 160 * 1024;
-        if (swiglu) {
-            if (four) return launch_fast<4, true>(a, sm_count, s);
-            if (two) return launch_fast<2, true>(a, sm_count, s);
-            return launch_fast<1, true>(a, sm_count, s);
+        // a row tile re-reads the weights
+        switch (q8_row_tile(a.M, a.K)) {
+            case 4: return swiglu ? launch_fast<4, true>(a, sm_count, s) : launch_fast<4, false>(a, sm_count, s);
+            case 2: return swiglu ? launch_fast<2, true>(a, sm_count, s) : launch_fast<2, false>(a, sm_count, s);
+            default: return swiglu ? launch_fast<1, true>(a, sm_count, s) : launch_fast<1, false>(a, sm_count, s);
         }
-        if (four) return launch_fast<4, false>(a, sm_count, s);
-        if (two) return launch_fast<2, false>(a, sm_count, s);
-        return launch_fast<1, false>(a, sm_count, s);
     }
     const size_t smem = (size_t)a.K * sizeof(float);
     if (smem > 200 * 1024) return cudaErrorInvalidValue;

@@ -316,3 +316,29 @@ def test_small_activations_beside_a_large_one(ctx, outlier, M):
     err = np.linalg.norm(ty.cpu().numpy() - truth) / np.linalg.norm(truth)
     assert err <= 1.15e-7, err
     W.close()
+
+
+@pytest.mark.parametrize("K,M,tensor", [(10240, 4, False), (10368, 4, True), (10368, 2, False), (12288, 3, True), (20480, 2, False),
+                                        (20608, 2, False), (20608, 3, True), (2176, 4, False), (256, 5, True)], ids=lambda v: str(v))
+def test_which_rows_the_row_kernels_keep(K, M, tensor):
+    """Two rows stay with the row kernels, three and four while one of their row tiles holds them; the tensor path shows by the
+    scratch it needs."""
+    import torch
+    import shainet_b200 as S
+    rng = np.random.default_rng(K + M)
+    N = 260
+    c = S.AttnContext(0)
+    q = rng.integers(-127, 128, (N, K)).astype(np.int8)
+    s = (0.001 * (0.5 + rng.random((N, K // 32)))).astype(np.float32)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    W = S.Q8Weight.from_quantized(c, q, s)
+    tx, ty = torch.from_numpy(x).cuda(), torch.empty((M, N), device="cuda")
+    torch.cuda.synchronize()
+    before = c.scratch_bytes()
+    W.gemv_dev(tx.data_ptr(), ty.data_ptr(), M)
+    c.sync()
+    assert (c.scratch_bytes() > before) == tensor
+    truth = x.astype(np.float64) @ (q.astype(np.float64) * s.astype(np.float64).repeat(32, 1)).T
+    assert rel_err(ty.cpu().numpy(), truth) <= DECODE_TOL
+    W.close()
+    c.close()
