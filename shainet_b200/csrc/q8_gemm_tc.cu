@@ -647,8 +647,10 @@ int token_tile(int M, int cap) {
     return nt < cap ? nt : cap;
 }
 
-// Cycles one 32-input block of a pair's tile takes: the tensor pipe at 128 tokens, the convert and accumulating warps below.
-double block_cycles(int nt) { return nt >= 128 ? 450.0 : nt >= 64 ? 330.0 : 260.0; }
+// What one 32-input block of a pair's tile takes, us: at 128 tokens the hand-overs over three accumulators, the convert and
+// accumulating warps below (fitted, with the constants of the plan, to 660 timed products of 512 to 9216 inputs, 2048 to 16384 outputs
+// and 8 to 4096 tokens, tiles and splits varied; the plan is on average 0.4 % slower than the best of them).
+double block_us(int nt) { return nt >= 128 ? 0.43 : nt >= 64 ? 0.32 : nt >= 32 ? 0.29 : 0.27; }
 
 }  // namespace
 
@@ -672,9 +674,9 @@ Q8GemmPlan q8_gemm_plan(int M, int K, int n0, int n1, int sm_count) {
         const long long tiles = (long long)n_tiles * t_tiles;
         for (int z = 1; z <= std::min(groups, 16); ++z) {
             const double waves = (double)((tiles * z + pairs - 1) / pairs);
-            // an item's blocks, its start-up and its stores; then the splits written and read back (bytes at 3.5 KB per cycle)
-            const double t = waves * (std::ceil((double)groups / z) * 4 * block_cycles(nt) + 900.0) +
-                             (z > 1 ? 2500.0 + 2.0 * z * (double)M * (n0 + n1) * 4 / 3500.0 : 0.0);
+            // an item's blocks, its start-up and its stores; then the splits written and read back
+            const double t = waves * (std::ceil((double)groups / z) * 4 * block_us(nt) + 0.9) +
+                             (z > 1 ? 2.5 + 0.63e-6 * z * (double)M * (n0 + n1) * 4 : 0.0);
             if (t < best_t) {
                 best_t = t;
                 best = Q8GemmPlan{nt, z};
