@@ -234,7 +234,7 @@ int pick_kernel(const HeadShape& hs, int batch, int T, unsigned flags, Kernel* o
     }
     if ((flags & SHAINET_ATTN_F_UNFUSED) && sk_ok && T <= SPLITK_MAX_T) *out = Kernel::SplitK;
     else if (tc_ok && T >= TENSOR_MIN_T) *out = Kernel::Tensor;
-    else *out = attn_rows_supported(hs) && (long long)batch * T <= 65535 ? Kernel::Rows : Kernel::Generic;
+    else *out = attn_rows_supported(hs) && (long long)batch * attn_rows_tiles(hs, T) <= 65535 ? Kernel::Rows : Kernel::Generic;
     return SHAINET_ATTN_OK;
 }
 

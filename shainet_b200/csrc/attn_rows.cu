@@ -430,14 +430,25 @@ int rows_ctas(int bm) {
 
 bool attn_rows_supported(const HeadShape& hs) { return hs.head_dim == 64 || hs.head_dim == 128; }
 
-AttnRowsPlan attn_rows_plan(const HeadShape& hs, int batch, int T, long long total_visible, int max_visible, int kv_elem_bytes, int sm_count) {
-    // rows per CTA: the tile that costs least, a 32- or 16-row tile paying for its shared-memory reads (fewer
-    // multiply-adds per operand load)
-    const int R = T * (hs.num_heads / hs.num_kv_heads);
+namespace {
+// Rows per CTA: the tile that costs least, a 32- or 16-row tile paying for its shared-memory reads (fewer multiply-adds per operand load)
+int tile_rows(int R) {
     auto cost = [&](int bm) { return (double)((R + bm - 1) / bm) * bm * (bm == 64 ? 1.0 : bm == 32 ? 1.2 : 1.7); };
-    AttnRowsPlan p{64, 64, 1};
+    int best = 64;
     for (int bm : {32, 16})
-        if (cost(bm) < cost(p.bm)) p.bm = bm;
+        if (cost(bm) < cost(best)) best = bm;
+    return best;
+}
+}  // namespace
+
+int attn_rows_tiles(const HeadShape& hs, int T) {
+    const int R = T * (hs.num_heads / hs.num_kv_heads), bm = tile_rows(R);
+    return (R + bm - 1) / bm;
+}
+
+AttnRowsPlan attn_rows_plan(const HeadShape& hs, int batch, int T, long long total_visible, int max_visible, int kv_elem_bytes, int sm_count) {
+    const int R = T * (hs.num_heads / hs.num_kv_heads);
+    AttnRowsPlan p{tile_rows(R), 64, 1};
     const int ctas_sm = hs.head_dim == 64 ? (kv_elem_bytes == 2 ? rows_ctas<64, 2>(p.bm) : rows_ctas<64, 4>(p.bm))
                                           : (kv_elem_bytes == 2 ? rows_ctas<128, 2>(p.bm) : rows_ctas<128, 4>(p.bm));
     // as many slices as fill the SMs once, each a whole number of 64-position tiles

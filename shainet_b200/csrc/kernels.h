@@ -147,6 +147,7 @@ struct AttnRowsPlan {
     int max_splits;
 };
 bool attn_rows_supported(const HeadShape& hs);
+int attn_rows_tiles(const HeadShape& hs, int T);   // query-row tiles per sequence and kv head; those of a batch lie along grid.z
 AttnRowsPlan attn_rows_plan(const HeadShape& hs, int batch, int T, long long total_visible, int max_visible, int kv_elem_bytes, int sm_count);
 cudaError_t launch_attn_rows(const AttnArgs& a, int bm, int kv_elem_bytes, cudaStream_t s);
 
