@@ -234,36 +234,45 @@ __global__ void __launch_bounds__(AR<HD, BM, ES>::THREADS, AR<HD, BM, ES>::CTAS)
             __syncwarp();
             // O += P V, four positions at a time.  In an edge tile a row stops at the last position it sees: what lies behind is the V
             // row of a later token, or of an earlier tile where this one is short, and zero times an infinity would be NaN.
-            auto pv = [&](auto checked) {
-                int seen[4];   // positions of this warp's strip that the row sees
+            // Only the few positions that some of the warp's eight rows see and others do not are checked row by row.
+            int kfull = C::KW, kend = C::KW, seen[4];   // positions of this warp's strip that all its rows, that any of them, that a row sees
+            if (edge) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) seen[i] = min(last[i] + 1, k1) - (k0 + t * C::BN + wk * C::KW);
-#pragma unroll 2
-                for (int k = 0; k < C::KW; k += 4) {
-                    float4 p4[4];
+                for (int i = 0; i < 4; ++i) seen[i] = min(C::KW, min(last[i] + 1, k1) - (k0 + t * C::BN + wk * C::KW));
+                kfull = max(0, __shfl_sync(FULL, seen[0], 0)) & ~3;
+                kend = __shfl_sync(FULL, seen[3], 31);
+            }
+            auto pv = [&](int k, auto checked) {
+                float4 p4[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) p4[i] = *reinterpret_cast<const float4*>(pw + (ty * 4 + i) * C::P_STRIDE + k);
+                for (int i = 0; i < 4; ++i) p4[i] = *reinterpret_cast<const float4*>(pw + (ty * 4 + i) * C::P_STRIDE + k);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        ulonglong2 vv[C::CT];
+                for (int kk = 0; kk < 4; ++kk) {
+                    ulonglong2 vv[C::CT];
 #pragma unroll
-                        for (int c = 0; c < C::CT; ++c) vv[c] = four<ES>(vs + ((size_t)(k + kk) * HD + c * 64 + tx * 4) * ES);
+                    for (int c = 0; c < C::CT; ++c) vv[c] = four<ES>(vs + ((size_t)(k + kk) * HD + c * 64 + tx * 4) * ES);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            if (decltype(checked)::value && k + kk >= seen[i]) continue;
-                            const float p = kk == 0 ? p4[i].x : kk == 1 ? p4[i].y : kk == 2 ? p4[i].z : p4[i].w;
-                            const f32x2 pp = ar_pack(p, p);
+                    for (int i = 0; i < 4; ++i) {
+                        if (decltype(checked)::value && k + kk >= seen[i]) continue;
+                        const float p = kk == 0 ? p4[i].x : kk == 1 ? p4[i].y : kk == 2 ? p4[i].z : p4[i].w;
+                        const f32x2 pp = ar_pack(p, p);
 #pragma unroll
-                            for (int c = 0; c < C::CT; ++c) {
-                                o[i][2 * c] = ar_fma(pp, vv[c].x, o[i][2 * c]);
-                                o[i][2 * c + 1] = ar_fma(pp, vv[c].y, o[i][2 * c + 1]);
-                            }
+                        for (int c = 0; c < C::CT; ++c) {
+                            o[i][2 * c] = ar_fma(pp, vv[c].x, o[i][2 * c]);
+                            o[i][2 * c + 1] = ar_fma(pp, vv[c].y, o[i][2 * c + 1]);
                         }
                     }
                 }
             };
-            if (edge) pv(std::true_type{});
-            else pv(std::false_type{});
+            if (!edge) {
+#pragma unroll 2
+                for (int k = 0; k < C::KW; k += 4) pv(k, std::false_type{});
+            } else {
+#pragma unroll 2
+                for (int k = 0; k < kfull; k += 4) pv(k, std::false_type{});
+#pragma unroll 1
+                for (int k = kfull; k < kend; k += 4) pv(k, std::true_type{});
+            }
             __syncwarp();   // the strip is rewritten in the next tile
             if (lane == 0) mbar_arrive(&empty[s]);
         }
