@@ -104,9 +104,9 @@ int shainet_attn_kv_create(shainet_attn_ctx* ctx, shainet_attn_kv** out, int num
  * and attention - still fp32 arithmetic, fp32 q, fp32 output - runs over the rounded
  * rows, the new token's own row included.  The result is therefore what the F32 path
  * gives on a cache whose rows were rounded that way, not what the reference gives on
- * unrounded rows.  Every entry that takes a cache accepts either format (single-token
- * decode and batched decode read bfloat16 directly; the other kernels read an fp32 image
- * of the rows that the context keeps as scratch) except shainet_attn_kv_device_ptrs
+ * unrounded rows.  Every entry that takes a cache accepts either format (decode, batched
+ * decode and calls of up to 63 new tokens at head_dim 64 and 128 read bfloat16 directly; the other
+ * kernels read an fp32 image of the rows that the context keeps as scratch) except shainet_attn_kv_device_ptrs
  * and batched decode with a kernel-forcing flag, which answer
  * SHAINET_ATTN_E_UNSUPPORTED.  kv_export widens exactly; kv_import and kv_fill_normal round. */
 #define SHAINET_ATTN_KV_F32 0

@@ -1026,8 +1026,8 @@ int shainet_attn_forward_host(shainet_attn_ctx* ctx, shainet_attn_kv* kv, const 
         CU(cudaMemcpyAsync(dk, k_new, kn * sizeof(float), cudaMemcpyHostToDevice, s));
         CU(cudaMemcpyAsync(dv, v_new, kn * sizeof(float), cudaMemcpyHostToDevice, s));
     }
-    // One decode token through the fused kernel: its merging CTAs store the few result
-    // rows straight into the pinned (device-visible) host buffer, which saves the
+    // One decode token through the fused kernel (or, at sixteen query heads per kv head, the row
+    // tiles): its merging CTAs store the few result rows straight into the pinned (device-visible) host buffer, which saves the
     // device-to-host copy operation and its latency.
     const bool direct_out = small && T == 1 && splitk_supported(kv->hs) &&
                             !(flags & (SHAINET_ATTN_F_GENERIC | SHAINET_ATTN_F_UNFUSED | SHAINET_ATTN_F_TENSOR));

@@ -781,7 +781,7 @@ cudaError_t launch_pf(const AttnArgs& a, cudaStream_t s) {
 }
 
 template <int HD>
-cudaError_t launch_pf_pair128(const AttnArgs& a, cudaStream_t s) {
+cudaError_t launch_pf_pair(const AttnArgs& a, cudaStream_t s) {
     using C = PFP<HD>;
     static unsigned long long configured = 0;
     int dev = 0;
@@ -829,10 +829,10 @@ cudaError_t launch_pf_pair128(const AttnArgs& a, cudaStream_t s) {
 template <int HD>
 cudaError_t launch_pf_any(const AttnArgs& a, cudaStream_t s) {
     // Even group size: two query heads of one kv head per pair of CTAs.  At head_dim 128 the pair halves the operand reads
-    // (0.70 against 0.98 ms for 8192 tokens of the Qwen3-8B shape); at head_dim 64 the two kernels are level on long prompts
+    // (0.69 against 0.87 ms for 8192 tokens of the Qwen3-8B shape); at head_dim 64 the two kernels are level on long prompts
     // (0.543 against 0.547 ms for 8192 tokens of the LLaMA-3.2-1B shape) and the pair, whose tile is half as large, is ahead
-    // where the row tiles do not fill the GPU (500 tokens over 3500: 45 against 72 us).
-    if ((a.hs.num_heads / a.hs.num_kv_heads) % 2 == 0 && !a.prefill_one_cta) return launch_pf_pair128<HD>(a, s);
+    // where the row tiles do not fill the GPU (500 tokens over 3500: 45 against 72 us).  There both give the same bits.
+    if ((a.hs.num_heads / a.hs.num_kv_heads) % 2 == 0 && !a.prefill_one_cta) return launch_pf_pair<HD>(a, s);
     return launch_pf<HD>(a, s);
 }
 

@@ -1,8 +1,8 @@
 // Q8_0 weight times several activation rows on the 5th-generation tensor cores (tcgen05), sm_100a: the projections and
 // FFN matrices of a prompt (or of any call with more than one new token).
 //
-// Replaces the reference's gemm_q8_f32_kernel (src/shainet/native/cuda_kernels.cu:581-629) for M > 1 and, through the
-// small kernels around it, the host loops between the projections (rms_norm.cr:18-37, swiglu_ff.cr:76-91,
+// Replaces the reference's gemm_q8_f32_kernel (src/shainet/native/cuda_kernels.cu:581-629) for several rows in the library's own
+// entries (the symbol gemm_q8_f32 has no scratch and keeps the row tiles) and, through the small kernels around it, the host loops between the projections (rms_norm.cr:18-37, swiglu_ff.cr:76-91,
 // llama_block.cr:189-196), with the single-row kernels' precision:
 //
 //  * the int8 weights are exact in bfloat16;
@@ -22,8 +22,8 @@
 //
 // Bounds.  The tensor core multiplies 4096 pairs per cycle and SM, but an MMA of 16 inputs takes at least about 64
 // cycles, however few its columns (the 128 rows of A have to pass).  At 128 tokens the three planes are three passes: 384
-// cycles per 32-input block, 0.2 us; what a block takes is 0.43 us, the hand-overs between convert, MMA and accumulating warps
-// over the three accumulators that tensor memory has room for.  At 64 tokens there is room for six.  With up to 32 tokens the planes lie
+// cycles per 32-input block; a block takes 760 (at 1.64 GHz, which six MMAs a block leave of the clock: 0.43 us).  72 % of the issue
+// slots go to the converting and accumulating warps and their waits over the three accumulators that tensor memory has room for.  At 64 tokens there is room for six.  With up to 32 tokens the planes lie
 // side by side as 3 NT columns of one pass, and the accumulating warps add the three columns of a token; the launch is then
 // bound by the convert warps and the contraction is split over the pairs (split-K) until they are all busy.
 // Measured, planes and split sums included: 4096 x 2048 -> 16384 in 777 us (row tiles of four on the CUDA cores 20.7 ms),
@@ -647,8 +647,8 @@ int token_tile(int M, int cap) {
     return nt < cap ? nt : cap;
 }
 
-// What one 32-input block of a pair's tile takes, us: at 128 tokens the hand-overs over three accumulators, the convert and
-// accumulating warps below (fitted, with the constants of the plan, to 660 timed products of 512 to 9216 inputs, 2048 to 16384 outputs
+// What one 32-input block of a pair's tile takes, us: at every width the issue slots of the convert and accumulating
+// warps first (fitted, with the constants of the plan, to 660 timed products of 512 to 9216 inputs, 2048 to 16384 outputs
 // and 8 to 4096 tokens, tiles and splits varied; the plan is on average 0.4 % slower than the best of them).
 double block_us(int nt) { return nt >= 128 ? 0.43 : nt >= 64 ? 0.32 : nt >= 32 ? 0.29 : 0.27; }
 

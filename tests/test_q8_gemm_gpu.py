@@ -29,7 +29,7 @@ def test_several_rows_against_f64(ctx, K, N, M):
     rng = np.random.default_rng(K + 3 * N + 7 * M)
     q = rng.integers(-128, 128, (N, K)).astype(np.int8)
     s = (0.001 * (0.5 + rng.random((N, K // 32)))).astype(np.float32)
-    # activations over thirty binary orders of magnitude: every bit of every one of them counts
+    # activations over thirty binary orders of magnitude (the error is normalised by the largest output here)
     x = (rng.standard_normal((M, K)) * np.exp2(rng.integers(-30, 1, (M, K)))).astype(np.float32)
     x[:, ::7] = rng.standard_normal((M, (K + 6) // 7)).astype(np.float32)
     W = S.Q8Weight.from_quantized(ctx, q, s)
@@ -38,7 +38,7 @@ def test_several_rows_against_f64(ctx, K, N, M):
     ty = torch.full((M + 1, N), float("nan"), device=dev)
     st = torch.cuda.Stream()
     torch.cuda.synchronize()
-    for stream in (st.cuda_stream, None):   # two streams share the context's scratch
+    for stream in (st.cuda_stream, None):   # on a caller's stream, then on the context's, over the same output
         W.gemv_dev(tx.data_ptr(), ty.data_ptr(), M, stream)
     torch.cuda.synchronize()
     ctx.sync()
