@@ -392,7 +392,7 @@ struct PFP {
     // At head_dim 64 a step is summed as the one-CTA kernel sums its two 64-position blocks, bit for bit: the running maximum
     // follows block after block (the probabilities, and with them their TF32 truncation, depend on it: with one
     // maximum per 128 positions results moved by 2e-4 of themselves), and so does the row sum.  500 tokens over 3500 bfloat16
-    // rows of the LLaMA-3.2-1B shape: 53 us a layer, 52 with one maximum.
+    // rows of the LLaMA-3.2-1B shape: 52.6 us a layer, 51.9 with one maximum.
     static constexpr bool BLOCKS64 = HD == 64;
     // [parity][half][row] row maxima, and with BLOCKS64 the sum of the half's probabilities in the step before; reused for the row sums
     static constexpr int XCHG_BYTES = 2 * 2 * BM * (BLOCKS64 ? 8 : 4);
@@ -569,11 +569,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const uint32_t oa = tmem + lane_addr + C::TMEM_O + half * (HD / 2);   // this thread's half of the output columns
         const uint32_t p_leader = map_to_cta(smem_u32(&p_full[0]), 0u);   // the leader's p_full[0]; the others follow at 8 bytes
         float m = -INFINITY, l = 0.0f;
-        // BLOCKS64: this half's sum of the step before (exchanged one step late, with the maxima), the factor between the sums
-        // of its two blocks, and whether there is one
-        float part = 0.0f, l_alpha = 1.0f;
-        bool second = false;
-        auto add_step = [&](float other) { l = (l + (half ? other : part)) * l_alpha + (half ? part : other); };
+        float part = 0.0f;   // BLOCKS64: this half's sum of the step before, exchanged one step late with the maxima
+        auto add_step = [&](float other) { l = (l + (half ? other : part)) + (half ? part : other); };
         bool ok = true;
         for (int j = 0; j < n; ++j) {
             const int b = j % SB;
@@ -599,7 +596,6 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             bool o_seen = j == 0;
             bool rescale;                       // of the accumulator, by alpha0 and then alpha1
             float alpha0 = 1.0f, alpha1 = 1.0f;
-            float my_m;                         // the maximum this thread's probabilities are taken against
             if constexpr (C::BLOCKS64) {
                 float2* xm = reinterpret_cast<float2*>(xchg) + (size_t)(j & 1) * 2 * C::BM;
                 xm[half * C::BM + r] = make_float2(mx, part);
@@ -608,26 +604,24 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
                 const float2 other = xm[(half ^ 1) * C::BM + r];
                 add_step(other.y);
                 // identical in both halves; where the larger of the two blocks' maxima asks for no rescaling, neither block does
-                second = false;
                 rescale = __any_sync(0xffffffffu, fmaxf(mx, other.x) * sl2 - m > C::RESCALE_STEP);   // always on the first step (m = -inf)
-                my_m = m;
                 if (rescale) {
                     const float m_first = fmaxf(m, (half ? other.x : mx) * sl2);
                     if (__any_sync(0xffffffffu, m_first - m > C::RESCALE_STEP)) {
                         alpha0 = ex2_approx(m - m_first);
                         m = m_first;
                         l *= alpha0;
-                        my_m = m;
                     }
+                    // Both blocks meet in one product: where the second one asks for a rescaling of its own the first one's probabilities
+                    // are taken against its maximum too, not rescaled in the accumulator as the one-CTA kernel does it (the one
+                    // place where the two are not bit for bit alike).
                     const float m_second = fmaxf(m, (half ? mx : other.x) * sl2);
-                    second = __any_sync(0xffffffffu, m_second - m > C::RESCALE_STEP);
-                    if (second) {
+                    if (__any_sync(0xffffffffu, m_second - m > C::RESCALE_STEP)) {
                         alpha1 = ex2_approx(m - m_second);
                         m = m_second;
-                        if (half) my_m = m;
+                        l *= alpha1;
                     }
                 }
-                l_alpha = alpha1;
             } else {
                 float* xm = xchg + (size_t)(j & 1) * 2 * C::BM;
                 xm[half * C::BM + r] = mx;
@@ -641,7 +635,6 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
                     m = m_cand;
                     l *= alpha0;
                 }
-                my_m = m;
             }
             if (rescale && j > 0) {
                 if (!(ok = mbar_wait(o_done, (j - 1) & 1, a.status, 60))) break;
@@ -664,8 +657,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             float sum0 = 0.0f, sum1 = 0.0f;
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
-                const float p0 = ex2_approx(fmaf(__uint_as_float(s0[c]), sl2, -my_m));
-                const float p1 = ex2_approx(fmaf(__uint_as_float(s1[c]), sl2, -my_m));
+                const float p0 = ex2_approx(fmaf(__uint_as_float(s0[c]), sl2, -m));
+                const float p1 = ex2_approx(fmaf(__uint_as_float(s1[c]), sl2, -m));
                 s0[c] = __float_as_uint(p0);
                 s1[c] = __float_as_uint(p1);
                 sum0 += p0;
@@ -673,15 +666,6 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             }
             if constexpr (C::BLOCKS64) {
                 part = sum0 + sum1;
-                // Both blocks meet in one product.  The first one's probabilities take the second one's rescaling here, where the
-                // one-CTA kernel has it in the accumulator (the one place where the two are not bit for bit alike).
-                if (second && half == 0) {
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) {
-                        s0[c] = __float_as_uint(__uint_as_float(s0[c]) * alpha1);
-                        s1[c] = __float_as_uint(__uint_as_float(s1[c]) * alpha1);
-                    }
-                }
             } else {
                 l += sum0 + sum1;
             }

@@ -166,8 +166,8 @@ def test_pair_of_ctas_at_head_dim_64(ctx, G, T, pre):
 @pytest.mark.parametrize("rising", [64, 128, 192], ids=lambda v: str(v))
 def test_pair_of_ctas_at_head_dim_64_with_rising_scores(ctx, rising):
     """Scores whose maximum jumps at a block of 64 positions, the first or the second one of a step: the accumulator and the
-    sums are rescaled between the blocks.  Where it is the second one the probabilities of the first are rescaled before the
-    tensor core cuts them to TF32 and not after: 2^-11 of each, so the two kernels agree within that tolerance."""
+    sums are rescaled between the blocks.  Where it is the second one the probabilities of the first are cut to TF32 against another
+    maximum than in the one-CTA kernel: 2^-11 of each, so the two kernels agree within that tolerance."""
     import shainet_b200 as S
     shape = dict(H=4, KV=2, hd=64, theta=10000.0)
     rng = np.random.default_rng(rising)
