@@ -180,8 +180,8 @@ int planes_acquire(shainet_attn_ctx* ctx, cudaStream_t s) {
     if (ctx->planes_in_use) return SHAINET_ATTN_OK;
     if (ctx->planes_pending) {
         unsigned long long id = 0;
-        CU(cudaStreamGetId(s, &id));
-        if (id != ctx->planes_stream) CU(cudaStreamWaitEvent(s, ctx->planes_ev, 0));
+        const bool same = cudaStreamGetId(s, &id) == cudaSuccess && id == ctx->planes_stream;
+        if (!same) CU(cudaStreamWaitEvent(s, ctx->planes_ev, 0));
     }
     ctx->planes_in_use = true;
     return SHAINET_ATTN_OK;
